@@ -250,11 +250,13 @@ int ysg_set_solver(ysg_handle *h, int which);
  * consecutive frequencies) ordered by estimated cost; 1 = lists of 32
  * entries (the spheroidal and the toroidal part of each pair) of equal code
  * path and near-equal exact step-count cost (a count-only pass and a sort
- * before the solve); 2 = the same lists in two concurrent launches, the
- * spheroidal parts and the toroidal parts (a small-slab, higher-occupancy
- * kernel on a second stream); -1
- * (default) = autotuned: the first time a workload signature is seen, the
- * solve stage runs once with each schedule and the fastest is kept.
+ * before the solve); 2 = the spheroidal, toroidal and radial parts in
+ * concurrent launches: by groups of degrees of one frequency that share a
+ * radial walk when every event has its source and receivers above the core,
+ * else the lists of 1 in two launches (the toroidal parts by a small-slab,
+ * higher-occupancy kernel); -1 (default) = 2 where it solves by groups, else
+ * autotuned: the first time a workload signature is seen, the solve stage
+ * runs once with each schedule and the fastest is kept.
  * Results do not depend on the schedule beyond rounding. */
 int ysg_set_schedule(ysg_handle *h, int sched);
 

@@ -151,7 +151,8 @@ class Engine:
 
     def set_schedule(self, sched: int) -> None:
         """Batched-solver schedule: 0 tiles, 1 cost-sorted pair lists, 2 the same lists
-        as a spheroidal and a toroidal launch, -1 autotuned."""
+        as a spheroidal and a toroidal launch (by groups of degrees sharing a radial
+        walk, for sources and receivers above the core), -1 chosen or autotuned."""
         N.check(N.lib().ysg_set_schedule(self.h, sched), "set_schedule")
 
     def last_schedule(self) -> tuple[int, list[float]]:

@@ -37,6 +37,7 @@ SOURCES = [
     CSRC / "capi.cu",
     CSRC / "k_solve_plain.cu",
     CSRC / "k_solve_batched.cu",
+    CSRC / "k_solve_group.cu",
     CSRC / "k_solve_tangent.cu",
     CSRC / "k_solve_adjoint.cu",
     CSRC / "k_schedule.cu",

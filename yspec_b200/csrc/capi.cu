@@ -137,6 +137,15 @@ struct ysg_handle {
     DevBuf offs, keys0, keys1, vals0, vals1, sort_tmp;
     DevBuf poff, pfx;                // per-frequency step table of the cost model (rows, table)
     long long nrows = 0;             // frequencies of the active slots
+    bool pairs_ready = false;        // the pair schedule's buffers fit the active slots
+    // solves by groups of degrees (k_solve_group.cu): item offsets per kind
+    // and event, order work space per kind, item counters
+    DevBuf tt, goff, gorder[NGROUP], gcounter;
+    long long gitems[NGROUP] = {};
+    int gblocks[NGROUP][NGROUP_FORM] = {};   // resident grid per kind and form
+    int gform[NGROUP] = {};          // form of the kernel per kind for the active slots
+    bool model_groups = false;       // the model's core boundaries are double knots
+    bool groups = false;             // the active slots can be solved by groups
     int sched = -1;                  // batched-solver schedule; -1 = autotuned
     int cur_sched = 0;               // schedule of the next solve launch
     std::map<Signature, int> tuned;  // autotuner choices
@@ -318,23 +327,61 @@ int upload_items(ysg_handle* h, const std::vector<EventDev>& evs, const std::vec
     for (size_t e = 0; e < evs.size(); e++) poff[e + 1] = poff[e] + evs[e].nw;
     CK(h->poff.ensure(poff.size() * sizeof(long long)));
     CK(cudaMemcpyAsync(h->poff.p, poff.data(), poff.size() * sizeof(long long), cudaMemcpyHostToDevice, h->st));
-    CK(h->pfx.ensure(std::max<size_t>((size_t)poff.back() * ((size_t)h->hdr.nknot + 1) * sizeof(int), 16)));
     h->nrows = poff.back();
-    const size_t pb = (size_t)std::max<long long>(2 * np, 1) * sizeof(unsigned long long);
-    CK(h->keys0.ensure(pb));
-    CK(h->keys1.ensure(pb));
-    CK(h->vals0.ensure(pb));
-    CK(h->vals1.ensure(pb));
-    CK(h->sort_tmp.ensure(std::max<size_t>(pair_sort_tmp_bytes(np), 16)));
+    // item lists of the group solver
+    std::vector<long long> goff((size_t)NGROUP * (evs.size() + 1), 0);
+    h->groups = h->solver == 1 && h->model_groups;
+    for (int k = 0; k < NGROUP && h->groups; k++) {
+        long long* o = &goff[(size_t)k * (evs.size() + 1)];
+        // the wide form where its items fill the GPU, else the narrow one
+        for (int form = 0; form < NGROUP_FORM; form++) {
+            if (h->gblocks[k][form] == 0) h->gblocks[k][form] = group_blocks(k, form);
+            if (h->gblocks[k][form] == 0) return YSG_ERR_CUDA;
+            const int width = group_form_width(k, form);
+            for (size_t e = 0; e < evs.size(); e++)
+                o[e + 1] = o[e] + group_items(evs[e].lmin, evs[e].lmax, evs[e].nw, evs[e].grav, k, width);
+            h->gform[k] = form;
+            if (o[evs.size()] >= h->gblocks[k][form]) break;
+        }
+        h->gitems[k] = o[evs.size()];
+        h->groups = h->groups && h->gitems[k] < (1ll << 31);
+    }
+    for (const EventDev& d : evs) h->groups = h->groups && d.is > h->hdr.noc && d.ir > h->hdr.noc;
+    if (h->groups) {
+        CK(h->goff.ensure(goff.size() * sizeof(long long)));
+        CK(h->gcounter.ensure(NGROUP * sizeof(unsigned long long)));
+        CK(cudaMemcpyAsync(h->goff.p, goff.data(), goff.size() * sizeof(long long), cudaMemcpyHostToDevice, h->st));
+        for (int k = 0; k < NGROUP; k++) {
+            if (h->gitems[k] > h->gblocks[k][h->gform[k]]) CK(h->gorder[k].ensure(group_order_bytes(h->gitems[k])));
+        }
+        h->h2d += (double)(goff.size() * sizeof(long long));
+    }
     CK(cudaStreamSynchronize(h->st));
     h->h2d += (double)(evs.size() * sizeof(EventDev) + coefs.size() * sizeof(cd*) +
                        (off.size() + poff.size()) * sizeof(long long));
     h->npairs = np;
     h->nev_items = (int)evs.size();
+    h->pairs_ready = false;
     for (int v = 0; v < NSOLVE_KERNELS; v++) {
         if (h->solve_blocks[v] == 0) h->solve_blocks[v] = solve_kernel_blocks(v);
         if (h->solve_blocks[v] == 0) return YSG_ERR_CUDA;
     }
+    return YSG_OK;
+}
+
+// Buffers of the pair schedule (k_schedule.cu) for the active slots, sized
+// only when a pair list is about to be built: the group solver needs none.
+int ensure_pairs(ysg_handle* h)
+{
+    if (h->pairs_ready) return YSG_OK;
+    CK(h->pfx.ensure(std::max<size_t>((size_t)h->nrows * ((size_t)h->hdr.nknot + 1) * sizeof(int), 16)));
+    const size_t pb = (size_t)std::max<long long>(2 * h->npairs, 1) * sizeof(unsigned long long);
+    CK(h->keys0.ensure(pb));
+    CK(h->keys1.ensure(pb));
+    CK(h->vals0.ensure(pb));
+    CK(h->vals1.ensure(pb));
+    CK(h->sort_tmp.ensure(std::max<size_t>(pair_sort_tmp_bytes(h->npairs), 16)));
+    h->pairs_ready = true;
     return YSG_OK;
 }
 
@@ -460,10 +507,41 @@ int upload_time(ysg_handle* h, Slot& s, const ysg_time* tm, int nw)
 int fork_side(ysg_handle* h, int nside);
 int join_side(ysg_handle* h, int nside);
 
+// The solves of the active slots by groups of degrees: the l = 0 solves
+// (few, long chains) first on a side stream, then the spheroidal kernels,
+// the toroidal one beside them on another side stream; all write disjoint
+// coefficients.
+int enqueue_groups(ysg_handle* h)
+{
+    const int nev = h->nev_items;
+    // side 1 is left out: a single event's Legendre table runs there
+    CK(cudaEventRecord(h->fork_ev, h->st));
+    for (int i : {0, 2}) CK(cudaStreamWaitEvent(h->side[i], h->fork_ev, 0));
+    auto launch = [&](int kind, cudaStream_t st) {
+        int n = 0;
+        const cudaError_t e = launch_group(
+            kind, h->gform[kind], h->kn.as<Knot>(), h->sg.as<Seg>(), h->hdr_dev.as<ModelHdr>(), h->evdev.as<EventDev>(),
+            h->coefptr.as<cd*>(), h->goff.as<long long>() + (size_t)kind * (nev + 1), nev, h->gitems[kind],
+            h->tt.as<double>(), h->gorder[kind].p, h->gcounter.as<unsigned long long>() + kind,
+            h->work.as<unsigned long long>(), h->gblocks[kind][h->gform[kind]], &n, st);
+        h->launches += n;
+        return e;
+    };
+    CK(launch(GROUP_RAD, h->side[2]));
+    for (int k : {GROUP_SPH2, GROUP_SPH1, GROUP_SPH0}) CK(launch(k, h->st));
+    CK(launch(GROUP_TOR, h->side[0]));
+    for (int i : {0, 2}) {
+        CK(cudaEventRecord(h->join_ev[i], h->side[i]));
+        CK(cudaStreamWaitEvent(h->st, h->join_ev[i], 0));
+    }
+    return YSG_OK;
+}
+
 int enqueue_solve(ysg_handle* h, int nev)
 {
     CK(cudaMemsetAsync(h->work.p, 0, NSYS_COUNT * sizeof(unsigned long long), h->st));
     CK(cudaMemsetAsync(h->status.p, 0, sizeof(int), h->st));
+    if (h->solver == 1 && h->cur_sched == 2 && h->groups) return enqueue_groups(h);
     if (h->solver == 0) {
         for (int e = 0; e < nev; e++) {
             const Slot& s = h->slots[(size_t)e];
@@ -565,9 +643,15 @@ int resolve_schedule(ysg_handle* h, int nev)
         h->cur_sched = 0;
         return ensure_tiles(h, nev);
     }
+    // Schedule 2 by groups of degrees is the fastest form at every size it
+    // takes (k_solve_group.cu): chosen without trial runs.
+    if (h->groups && (h->sched < 0 || h->sched == 2)) {
+        h->cur_sched = 2;
+        return YSG_OK;
+    }
     if (h->sched >= 0) {
         h->cur_sched = h->sched;
-        return h->sched == 0 ? ensure_tiles(h, nev) : YSG_OK;
+        return h->sched == 0 ? ensure_tiles(h, nev) : ensure_pairs(h);
     }
     long long maxl = 0, maxw = 0;
     for (int e = 0; e < nev; e++) {
@@ -584,9 +668,10 @@ int resolve_schedule(ysg_handle* h, int nev)
     auto it = h->tuned.find(sig);
     if (it != h->tuned.end()) {
         h->cur_sched = it->second;
-        return it->second == 0 ? ensure_tiles(h, nev) : YSG_OK;
+        return it->second == 0 ? ensure_tiles(h, nev) : ensure_pairs(h);
     }
     int rc0 = ensure_tiles(h, nev);     // the trials include schedule 0
+    if (!rc0) rc0 = ensure_pairs(h);
     if (rc0) return rc0;
     // The first tuning of a handle runs each schedule once untimed: with lazy
     // module loading a kernel's first launch also loads its module on the
@@ -820,7 +905,10 @@ int prepare_single(ysg_handle* h, const ysg_event* ev)
         if (!rc) rc = resolve_schedule(h, 1);
         return rc;
     }
-    if (h->solver == 2) return upload_batch_items(h, 1);
+    if (h->solver == 2) {
+        rc = upload_batch_items(h, 1);
+        return rc ? rc : ensure_pairs(h);
+    }
     return YSG_OK;
 }
 
@@ -1042,10 +1130,11 @@ void ysg_destroy(ysg_handle* h)
     for (Slot& s : h->slots) s.release();
     for (DevBuf* b : {&h->kn, &h->sg, &h->hdr_dev, &h->offs, &h->keys0, &h->keys1, &h->vals0,
                       &h->vals1, &h->sort_tmp, &h->poff, &h->pfx, &h->work, &h->status, &h->items, &h->counter,
-                      &h->evdev, &h->coefptr, &h->dkn, &h->dsg, &h->ukn, &h->usg, &h->abasis,
+                      &h->evdev, &h->coefptr, &h->tt, &h->goff, &h->gcounter, &h->dkn, &h->dsg, &h->ukn, &h->usg, &h->abasis,
                       &h->about, &h->ascr, &h->acs0, &h->agout, &h->asbar, &h->acoefb, &h->agrad, &h->alogs})
         b->release();
     for (DevBuf& b : h->scratch) b.release();
+    for (DevBuf& b : h->gorder) b.release();
     for (auto& e : h->ev)
         if (e) cudaEventDestroy(e);
     for (int i = 0; i < ysg_handle::NSIDE; i++) {
@@ -1140,7 +1229,16 @@ int ysg_model_upload(ysg_handle* h, const ysg_model* m)
     CK(cudaMemcpyAsync(h->sg.p, seg.data(), seg.size() * sizeof(Seg), cudaMemcpyHostToDevice, h->st));
     CK(h->hdr_dev.ensure(sizeof(ModelHdr)));
     CK(cudaMemcpyAsync(h->hdr_dev.p, &hd, sizeof(ModelHdr), cudaMemcpyHostToDevice, h->st));
+    // sum of length / alpha below each knot: the walk's step count per 4 omega
+    std::vector<double> tt((size_t)n + 2, 0.0);
+    for (int i = 1; i < n; i++)
+        tt[(size_t)i + 1] = tt[(size_t)i] + (m->r[i] - m->r[i - 1]) / std::max(m->alpha[i - 1], m->alpha[i]);
+    tt[(size_t)n + 1] = tt[(size_t)n];
+    CK(h->tt.ensure(tt.size() * sizeof(double)));
+    CK(cudaMemcpyAsync(h->tt.p, tt.data(), tt.size() * sizeof(double), cudaMemcpyHostToDevice, h->st));
     CK(cudaStreamSynchronize(h->st));
+    // legs of different lanes meet at the core boundaries (k_solve_group.cu)
+    h->model_groups = m->noc < n && m->r[m->nic - 1] == m->r[m->nic] && m->r[m->noc - 1] == m->r[m->noc];
     h->hdr = hd;
     h->grav_host.assign(m->val[P_GRAV], m->val[P_GRAV] + n);
     h->r_host.assign(m->r, m->r + n);
@@ -1275,6 +1373,7 @@ int ysg_event_gradient(ysg_handle* h, const ysg_event* ev, const ysg_time* tm, c
     rc = upload_event(h, s, ev);
     if (!rc) rc = upload_time(h, s, tm, ev->nw);
     if (!rc) rc = upload_batch_items(h, 1);
+    if (!rc) rc = ensure_pairs(h);
     if (!rc) rc = ensure_units(h);
     if (rc) return rc;
     h->nactive = 1;
@@ -1593,6 +1692,7 @@ int ysg_batch_run(ysg_handle* h, int nev, const ysg_event* evs, const ysg_time* 
         if (rc) return rc;
     } else if (h->solver == 2) {
         int rc = upload_batch_items(h, nev);
+        if (!rc) rc = ensure_pairs(h);
         if (rc) return rc;
     }
     h->nactive = nev;

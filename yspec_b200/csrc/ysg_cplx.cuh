@@ -9,6 +9,15 @@
 #include <cuda_runtime.h>
 #include <math.h>
 
+// Division, modulus, square root and logarithm are inlined by default; a
+// file whose kernels run them outside their hot loops can keep one copy of
+// each instead (YSG_CPLX_CALLS), for its instruction footprint.
+#ifdef YSG_CPLX_CALLS
+#define YSG_CPLX_FN inline __noinline__
+#else
+#define YSG_CPLX_FN __forceinline__
+#endif
+
 namespace ysg {
 
 // 16-byte aligned so that a complex value moves with one 128-bit load or
@@ -27,7 +36,7 @@ __host__ __device__ __forceinline__ cd operator*(cd a, cd b)
 }
 __host__ __device__ __forceinline__ cd operator*(double s, cd a) { return cd{s * a.x, s * a.y}; }
 __host__ __device__ __forceinline__ cd operator*(cd a, double s) { return cd{a.x * s, a.y * s}; }
-__host__ __device__ __forceinline__ cd operator/(cd a, double s) { return cd{a.x / s, a.y / s}; }
+__host__ __device__ YSG_CPLX_FN cd operator/(cd a, double s) { return cd{a.x / s, a.y / s}; }
 __host__ __device__ __forceinline__ cd operator+(cd a, double s) { return cd{a.x + s, a.y}; }
 __host__ __device__ __forceinline__ cd operator+(double s, cd a) { return cd{s + a.x, a.y}; }
 __host__ __device__ __forceinline__ cd operator-(cd a, double s) { return cd{a.x - s, a.y}; }
@@ -36,7 +45,7 @@ __host__ __device__ __forceinline__ cd& operator+=(cd& a, cd b) { a.x += b.x; a.
 __host__ __device__ __forceinline__ cd& operator-=(cd& a, cd b) { a.x -= b.x; a.y -= b.y; return a; }
 
 // Smith's algorithm for a / b.
-__host__ __device__ __forceinline__ cd operator/(cd a, cd b)
+__host__ __device__ YSG_CPLX_FN cd operator/(cd a, cd b)
 {
     if (fabs(b.x) >= fabs(b.y)) {
         double r = b.y / b.x;
@@ -51,10 +60,10 @@ __host__ __device__ __forceinline__ cd operator/(cd a, cd b)
 __host__ __device__ __forceinline__ cd operator/(double s, cd b) { return cd{s, 0.0} / b; }
 
 __host__ __device__ __forceinline__ cd conj(cd a) { return cd{a.x, -a.y}; }
-__host__ __device__ __forceinline__ double cabs(cd a) { return hypot(a.x, a.y); }
+__host__ __device__ YSG_CPLX_FN double cabs(cd a) { return hypot(a.x, a.y); }
 __host__ __device__ __forceinline__ cd imul(cd a) { return cd{-a.y, a.x}; }   // i*a
 
-__host__ __device__ __forceinline__ cd csqrt(cd z)
+__host__ __device__ YSG_CPLX_FN cd csqrt(cd z)
 {
     if (z.x == 0.0 && z.y == 0.0) return cd{0.0, z.y};
     double t = sqrt((fabs(z.x) + hypot(z.x, z.y)) * 0.5);
@@ -62,6 +71,6 @@ __host__ __device__ __forceinline__ cd csqrt(cd z)
     return cd{fabs(z.y) / (2.0 * t), copysign(t, z.y)};
 }
 
-__host__ __device__ __forceinline__ cd clog(cd z) { return cd{log(hypot(z.x, z.y)), atan2(z.y, z.x)}; }
+__host__ __device__ YSG_CPLX_FN cd clog(cd z) { return cd{log(hypot(z.x, z.y)), atan2(z.y, z.x)}; }
 
 }  // namespace ysg

@@ -47,6 +47,27 @@ cudaError_t launch_solve_kernel(int kid, const Knot* kn, const Seg* sg, const Mo
                                 int item0, int item_end, int* counter, unsigned long long* work,
                                 int nblocks, cudaStream_t st);
 
+// K1 by groups of 32 degrees of one frequency (k_solve_group.cu), one list
+// of items per kind: the three gravity settings of the spheroidal solves
+// (GROUP_SPH0 + grav), the toroidal and the l = 0 ones.  For events with
+// the source and the receivers above the core.
+enum GroupKind { GROUP_SPH0 = 0, GROUP_SPH1, GROUP_SPH2, GROUP_TOR, GROUP_RAD, NGROUP };
+// Forms of a kind's kernel: 0 for lists that fill the GPU (128 degrees per
+// item), 1 for short ones (32 degrees per item).
+constexpr int NGROUP_FORM = 2;
+int group_form_width(int kind, int form);                               // degrees per item
+long long group_items(int lmin, int lmax, int nw, int grav, int kind, int width);   // items of an event
+int group_blocks(int kind, int form);                                   // resident grid, 0 on failure
+// Bytes of the ordering work space of a list (used when nitems exceeds the resident grid).
+size_t group_order_bytes(long long nitems);
+// off: items of the events before e (nev + 1 entries); tt (nknot + 1
+// entries): sum of length / alpha over the intervals below knot k; counter
+// is reset here.  *launched receives the kernels enqueued.
+cudaError_t launch_group(int kind, int form, const Knot* kn, const Seg* sg, const ModelHdr* mh, const EventDev* evs,
+                         cd* const* coefs, const long long* off, int nev, long long nitems, const double* tt,
+                         void* order_buf, unsigned long long* counter, unsigned long long* work, int resident,
+                         int* launched, cudaStream_t st);
+
 // Pair cost model and ordering for schedule 1 (k_schedule.cu).  off[e] is
 // the flat index of event e's first pair (off[nev] = npairs); keys and vals
 // are two pairs of npairs-element buffers; *sorted receives the buffer

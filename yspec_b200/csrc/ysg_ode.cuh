@@ -412,11 +412,14 @@ __device__ __forceinline__ FluidCoef fluid_amat(const Ctx& c, double rr)
 
 // ---------------------------------------------------------------------------
 // Right-hand sides.  Each system is a tag type with N components and f().
+// f takes any context C for which the system's *_amat(c, r) is declared:
+// Ctx evaluates the model at r (above), the group solver's lane contexts
+// (ysg_group.cuh) combine coefficients shared by the lanes of a warp.
 // ---------------------------------------------------------------------------
 struct TorSys {
     static constexpr int N = 2, CLS = 0;
-    template <class Out>
-    __device__ static __forceinline__ void f(const Ctx& c, double r, const mcplx* y, Out d)
+    template <class C, class Out>
+    __device__ static __forceinline__ void f(const C& c, double r, const mcplx* y, Out d)
     {
         TorCoef a = tor_amat(c, r);       // module_int.f90:168-184
         d[0] = cmac(a.t * y[0], a.k, y[1]);
@@ -426,8 +429,8 @@ struct TorSys {
 
 struct RadSys {
     static constexpr int N = 2, CLS = 1;
-    template <class Out>
-    __device__ static __forceinline__ void f(const Ctx& c, double r, const mcplx* y, Out d)
+    template <class C, class Out>
+    __device__ static __forceinline__ void f(const C& c, double r, const mcplx* y, Out d)
     {
         RadCoef a = rad_amat(c, r);       // module_int.f90:357-392
         d[0] = cmac(a.t * y[0], a.k, y[1]);
@@ -438,8 +441,8 @@ struct RadSys {
 // module_int.f90:818-871 sph_minors_solid_derivs
 struct MinorSolidG {
     static constexpr int N = 14, CLS = 6;
-    template <class Out>
-    __device__ static __forceinline__ void f(const Ctx& c, double r, const mcplx* m, Out d)
+    template <class C, class Out>
+    __device__ static __forceinline__ void f(const C& c, double r, const mcplx* m, Out d)
     {
         SolidCoef a = solid_amat<2>(c, r);
         mcplx a123 = a.t11 + (a.t22 + a.t33), a126 = a.t11 + (a.t22 - a.t33);
@@ -465,8 +468,8 @@ struct MinorSolidG {
 template <int KIND>
 struct MinorSolidNC {
     static constexpr int N = 5, CLS = 4;
-    template <class Out>
-    __device__ static __forceinline__ void f(const Ctx& c, double r, const mcplx* m, Out d)
+    template <class C, class Out>
+    __device__ static __forceinline__ void f(const C& c, double r, const mcplx* m, Out d)
     {
         SolidCoef a = solid_amat<KIND>(c, r);
         mcplx a11 = a.t11 + a.t22, a22 = a.t11 - a.t22;
@@ -481,8 +484,8 @@ struct MinorSolidNC {
 // module_int.f90:941-967 sph_minors_fluid_derivs
 struct MinorFluidG {
     static constexpr int N = 5, CLS = 5;
-    template <class Out>
-    __device__ static __forceinline__ void f(const Ctx& c, double r, const mcplx* m, Out d)
+    template <class C, class Out>
+    __device__ static __forceinline__ void f(const C& c, double r, const mcplx* m, Out d)
     {
         FluidCoef a = fluid_amat<2>(c, r);
         mcplx tp = a.t11 + a.t22, tm = a.t11 - a.t22;
@@ -498,8 +501,8 @@ struct MinorFluidG {
 template <int KIND>
 struct MinorFluidNC {
     static constexpr int N = 2, CLS = 2;
-    template <class Out>
-    __device__ static __forceinline__ void f(const Ctx& c, double r, const mcplx* m, Out d)
+    template <class C, class Out>
+    __device__ static __forceinline__ void f(const C& c, double r, const mcplx* m, Out d)
     {
         FluidCoef a = fluid_amat<KIND>(c, r);
         d[0] = cmac(a.t11 * m[0], a.k11, m[1]);
@@ -510,8 +513,8 @@ struct MinorFluidNC {
 // module_int.f90:1016-1057 sph_bvec_solid_derivs
 struct BvecSolidG {
     static constexpr int N = 14, CLS = 7;
-    template <class Out>
-    __device__ static __forceinline__ void f(const Ctx& c, double r, const mcplx* b, Out d)
+    template <class C, class Out>
+    __device__ static __forceinline__ void f(const C& c, double r, const mcplx* b, Out d)
     {
         SolidCoef a = solid_amat<2>(c, r);
         const mcplx t11 = a.t11, t12 = a.t12, k11 = a.k11, k22 = a.k22;
@@ -563,8 +566,8 @@ struct BvecSolidGTr {
         d[12] = cmsc(cmsc(cmac(cmac(cmac(s13 * k[2], s23, k[6]), (t11 + t33), k[12]), t21, k[13]), s11, k[4]), s12, k[8]);
         d[13] = cmsc(cmsc(cmac(cmac(cmac(s13 * k[3], s23, k[7]), t12, k[12]), (t22 + t33), k[13]), s12, k[4]), s22, k[8]);
     }
-    template <class Out>
-    __device__ static __forceinline__ void f(const Ctx& c, double r, const mcplx* k, Out d)
+    template <class C, class Out>
+    __device__ static __forceinline__ void f(const C& c, double r, const mcplx* k, Out d)
     {
         tr(solid_amat<2>(c, r), k, d);
     }
@@ -574,8 +577,8 @@ struct BvecSolidGTr {
 template <int KIND>
 struct BvecSolidNC {
     static constexpr int N = 4, CLS = 3;
-    template <class Out>
-    __device__ static __forceinline__ void f(const Ctx& c, double r, const mcplx* b, Out d)
+    template <class C, class Out>
+    __device__ static __forceinline__ void f(const C& c, double r, const mcplx* b, Out d)
     {
         SolidCoef a = solid_amat<KIND>(c, r);
         d[0] = cmsc(cmsc(cmsc(-(a.s11 * b[2]), a.s12, b[3]), a.t11, b[0]), a.t21, b[1]);
@@ -590,8 +593,8 @@ struct BvecSolidNC {
 template <int KIND>
 struct BvecSolidNCTr {
     static constexpr int N = 4, CLS = 3;
-    template <class Out>
-    __device__ static __forceinline__ void f(const Ctx& c, double r, const mcplx* k, Out d)
+    template <class C, class Out>
+    __device__ static __forceinline__ void f(const C& c, double r, const mcplx* k, Out d)
     {
         const SolidCoef a = solid_amat<KIND>(c, r);
         d[0] = cmsc(cmsc(-(a.t11 * k[0]), a.t12, k[1]), a.k11, k[2]);

@@ -53,6 +53,14 @@ __device__ __forceinline__ cd out_factor(int out, cd w)
     return out == 1 ? imul(w) : (out == 2 ? -(w * w) : mk(1.0));
 }
 
+// The rows of the spheroidal responses a pair's coefficients use (bit k for
+// row k): the potential (row 2) alone, or the two displacement rows, with
+// row 2 for the tilt and potential correction of the acceleration.
+__device__ __forceinline__ int spheroidal_rows(const EventDev& ev)
+{
+    return ev.pot ? 0x4 : ((ev.out == 2 && ev.cor != 0) ? 0x7 : 0x3);
+}
+
 }  // namespace ysg
 #endif  // YSG_SOLVERS_COMMON
 
@@ -669,19 +677,11 @@ __device__ inline void pair_radial(Ctx& c, const EventDev& ev, int j, mcplx* coe
     coef[2] = u3;
 }
 
-// l >= 2: toroidal part, yspec.f90:301-316 -> ww(1:5)
-__device__ inline void pair_toroidal(Ctx& c, const EventDev& ev, int l, int j, mcplx* ww)
+// ww(1:5) from the responses of tor_solver (yspec.f90:305-316); ytor is scaled in place
+__device__ inline void toroidal_coefs(const Ctx& c, const EventDev& ev, int l, cd w, mcplx (*ytor)[2], mcplx* ww)
 {
-    if (ev.pot) {                                     // toroidal motion carries no potential
-        for (int q = 0; q < 5; q++) ww[q] = mk(0.0);
-        return;
-    }
-    cd w = omega_of(ev, j);
-    set_l(c, l);
-    set_omega(c, w);
-    mcplx svt[5][2], ytor[2][2];
+    mcplx svt[5][2];
     source_vector_tor(c, ev.is, ev.rs, ev.mm, svt);
-    tor_solver(c, ev.rr, ev.rs, ev.ir, ev.is, ytor);
     if (ev.out != 0) {
         cd f = out_factor(ev.out, w);
         for (int a = 0; a < 2; a++)
@@ -692,32 +692,26 @@ __device__ inline void pair_toroidal(Ctx& c, const EventDev& ev, int l, int j, m
     for (int q = 0; q < 5; q++) ww[q] = (svt[q][0] * ytor[0][0] + svt[q][1] * ytor[0][1]) / zr;
 }
 
-// l >= 1: spheroidal part, yspec.f90:344-400 -> uu(1:5), vv(1:5)
-__device__ inline void pair_spheroidal(Ctx& c, const EventDev& ev, int l, int j, mcplx* uu, mcplx* vv)
+// l >= 2: toroidal part, yspec.f90:301-316 -> ww(1:5)
+__device__ inline void pair_toroidal(Ctx& c, const EventDev& ev, int l, int j, mcplx* ww)
 {
+    if (ev.pot) {                                     // toroidal motion carries no potential
+        for (int q = 0; q < 5; q++) ww[q] = mk(0.0);
+        return;
+    }
     cd w = omega_of(ev, j);
     set_l(c, l);
     set_omega(c, w);
-    alpha_steps(c);
-    mcplx ysph[kSphRows][4];
-    if (ev.grav == 2) {
-        // the rows of the responses used below: the potential (row 2) alone,
-        // or the two displacement rows, with row 2 for the tilt and
-        // potential correction of the acceleration
-        const int rows = ev.pot ? 0x4 : ((ev.out == 2 && ev.cor != 0) ? 0x7 : 0x3);
-        sph_solver_g(c, ev.rr, ev.rs, ev.ir, ev.is, ysph, rows);
-    } else {
-        mcplx yng[kNcRows][4];
-        if (ev.grav == 1) sph_solver_nc<1>(c, ev.rr, ev.rs, ev.ir, ev.is, yng);
-        else sph_solver_nc<0>(c, ev.rr, ev.rs, ev.ir, ev.is, yng);
-        for (int b = 0; b < 4; b++) {                  // yspec.f90:367-374
-            ysph[0][b] = yng[0][b];
-            ysph[1][b] = yng[1][b];
-            ysph[2][b] = mk(0.0);
-        }
-    }
-    // the source vectors depend on none of the solve's state: formed after
-    // it, they share no stack with the solver's minors
+    mcplx ytor[2][2];
+    tor_solver(c, ev.rr, ev.rs, ev.ir, ev.is, ytor);
+    toroidal_coefs(c, ev, l, w, ytor, ww);
+}
+
+// uu(1:5), vv(1:5) from the response rows 0-2 to the four source jumps
+// (yspec.f90:365-400); ysph is scaled in place
+__device__ inline void spheroidal_coefs(const Ctx& c, const EventDev& ev, int l, cd w, mcplx (*ysph)[4], mcplx* uu,
+                                        mcplx* vv)
+{
     mcplx svs[5][6];
     source_vector_sph(c, ev.is, ev.rs, ev.mm, svs);
     double zeta = (double)sqrtf((float)(l * (l + 1)));   // yspec.f90:255 (FP32)
@@ -762,6 +756,31 @@ __device__ inline void pair_spheroidal(Ctx& c, const EventDev& ev, int l, int j,
         vv[q] = (ysph[1][0] * svs[q][0] + ysph[1][1] * svs[q][1] + ysph[1][2] * svs[q][3] +
                  ysph[1][3] * svs[q][4]) / zr;
     }
+}
+
+// l >= 1: spheroidal part, yspec.f90:344-400 -> uu(1:5), vv(1:5)
+__device__ inline void pair_spheroidal(Ctx& c, const EventDev& ev, int l, int j, mcplx* uu, mcplx* vv)
+{
+    cd w = omega_of(ev, j);
+    set_l(c, l);
+    set_omega(c, w);
+    alpha_steps(c);
+    mcplx ysph[kSphRows][4];
+    if (ev.grav == 2) {
+        sph_solver_g(c, ev.rr, ev.rs, ev.ir, ev.is, ysph, spheroidal_rows(ev));
+    } else {
+        mcplx yng[kNcRows][4];
+        if (ev.grav == 1) sph_solver_nc<1>(c, ev.rr, ev.rs, ev.ir, ev.is, yng);
+        else sph_solver_nc<0>(c, ev.rr, ev.rs, ev.ir, ev.is, yng);
+        for (int b = 0; b < 4; b++) {                  // yspec.f90:367-374
+            ysph[0][b] = yng[0][b];
+            ysph[1][b] = yng[1][b];
+            ysph[2][b] = mk(0.0);
+        }
+    }
+    // the source vectors depend on none of the solve's state: formed after
+    // it, they share no stack with the solver's minors
+    spheroidal_coefs(c, ev, l, w, ysph, uu, vv);
 }
 
 }  // inline namespace
