@@ -7,7 +7,7 @@
 //   k_group_split   spheroidal with self-gravitation, 32 degrees per item, the
 //                   14 components split over NW warps
 //   k_group_tor     toroidal, a degree per lane, NL warps per item
-//   k_group_rad     l = 0, a thread per frequency
+//   k_group_rad     l = 0, a warp per frequency
 // Events with the source or a receiver in the core, where legs of different
 // lanes would run in different directions, take the pair lists of
 // k_solve_batched.cu instead.
@@ -44,7 +44,7 @@
 #include <algorithm>
 
 #include "ysg_kernels.h"
-#include "ysg_group.cuh"
+#include "ysg_radial.cuh"
 
 namespace ysg {
 namespace {
@@ -709,34 +709,47 @@ __global__ void __launch_bounds__(32 * NL, MINB) k_group_tor(GroupArgs a)
 }
 
 // ---------------------------------------------------------------------------
-// l = 0: a thread per frequency.
+// l = 0 (pair_radial of ysg_solvers.cuh): a warp per frequency (ysg_radial.cuh).
+// The chain of steps bounds it: a thread per frequency took 0.94 ms on an
+// event of 9,060 pairs (10 mHz), a warp 0.21 ms, beside spheroidal solves of
+// 0.92 ms; on one event of 300,000 pairs (220 knots, 40 mHz, deck with an
+// ocean) the solve stage went from 9.1 to 5.2 ms with it.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(32) k_group_rad(GroupArgs a)
 {
+    __shared__ RadMem M;
+    const int lane = threadIdx.x;
+    const long long it = blockIdx.x;
+    int lo = 0, hi = a.nev;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (a.off[mid] <= it) lo = mid;
+        else hi = mid;
+    }
+    const EventDev& ev = a.evs[lo];
+    const int j = ev.nw - (int)(it - a.off[lo]);
     Group g;
     group_ctx(g, a);
-    const long long it = (long long)blockIdx.x * 32 + threadIdx.x;
-    if (it < a.nitems) {
-        int lo = 0, hi = a.nev;
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (a.off[mid] <= it) lo = mid;
-            else hi = mid;
-        }
-        const EventDev& ev = a.evs[lo];
-        const int j = ev.nw - (int)(it - a.off[lo]);
-        g.c.ats = (double)ev.ats;
-        cd out[NCOEF];
-        pair_radial(g.c, ev, j, out);
-        cd* dst = a.coefs[lo] + (j - 1);
-        for (int q = 0; q < NCOEF; q++)
-            __stcs(reinterpret_cast<double2*>(dst + (size_t)q * ev.nw), make_double2(out[q].x, out[q].y));
-    }
-    for (int q = 0; q < NSYS; q++) {
-        unsigned long long v = g.c.nst[q];
-        for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(FULL, v, off);
-        if (threadIdx.x == 0 && v) atomicAdd(&a.work[q], v);
-    }
+    Ctx& c = g.c;
+    c.ats = (double)ev.ats;
+    set_l(c, 0);
+    set_omega(c, omega_of(ev, j));
+    alpha_steps(c);
+    cd sr0[2], yrad[2][2], ph[2] = {mk(0.0), mk(0.0)};
+    unsigned n = 0;
+    source_vector_rad(c, ev.is, ev.rs, ev.mm, sr0);
+    if (ev.grav != 0) rad_wg_warp(c, M, lane, ev.rr, ev.rs, yrad, ev.pot ? ph : nullptr, &n);
+    else if (!ev.pot) rad_ng_warp(c, M, lane, ev.rr, ev.rs, ev.ir, ev.is, yrad, &n);
+    cd u3;
+    if (ev.pot) u3 = (sr0[0] * ph[0] + sr0[1] * ph[1]) / ev.rr;     // no gravity, no potential
+    else u3 = (sr0[0] * yrad[0][0] + sr0[1] * yrad[0][1]) / ev.rr;
+    if (ev.out != 0) u3 = out_factor(ev.out, c.omega) * u3;
+    cd* dst = a.coefs[lo] + (j - 1);
+    if (lane < NCOEF)
+        __stcs(reinterpret_cast<double2*>(dst + (size_t)lane * ev.nw),
+               lane == 2 ? make_double2(u3.x, u3.y) : make_double2(0.0, 0.0));
+    n = __reduce_add_sync(FULL, n);
+    if (lane == 0 && n) atomicAdd(&a.work[RadSys::CLS], (unsigned long long)n);
 }
 
 // ---------------------------------------------------------------------------
@@ -874,7 +887,7 @@ cudaError_t launch_group(int kind, int form, const Knot* kn, const Seg* sg, cons
     GroupArgs a{kn, sg, mh, evs, coefs, off, nullptr, nev, nitems, counter, work};
     const GroupKernel k = group_kernel(kind, form);
     if (kind == GROUP_RAD) {
-        k_group_rad<<<(unsigned)((nitems + 31) / 32), 32, 0, st>>>(a);
+        k_group_rad<<<(unsigned)nitems, 32, 0, st>>>(a);
         *launched = 1;
         return cudaGetLastError();
     }

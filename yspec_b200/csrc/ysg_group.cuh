@@ -359,6 +359,7 @@ __device__ __forceinline__ int hi_abs(double x) { return __double2hiint(x) & 0x7
 // The walk of a group along yint's steps: 32 knot intervals at a time, one
 // per lane, and the steps of those intervals in batches of SB.
 struct Walk {
+    bool rev;                     // the steps in reverse order
     int i1, i2;
     double r1, r2;
     int q0, s0, total;            // next chunk of intervals; next step and steps of this chunk
@@ -366,8 +367,9 @@ struct Walk {
     double x, h;                  // the lane's interval: first radius, step
 };
 
-__device__ __forceinline__ void walk_init(Walk& w, int i1, int i2, double r1, double r2)
+__device__ __forceinline__ void walk_init(Walk& w, int i1, int i2, double r1, double r2, bool rev)
 {
+    w.rev = rev;
     w.i1 = i1;
     w.i2 = i2;
     w.r1 = r1;
@@ -375,22 +377,16 @@ __device__ __forceinline__ void walk_init(Walk& w, int i1, int i2, double r1, do
     w.q0 = w.s0 = w.total = 0;
 }
 
-// The points, step sizes and intervals of the next batch of steps (yint's,
-// or with TR in reverse order) into shared memory; returns its steps, 0 at
-// the end of the walk.  The warps of a group call it together: one copy in
-// the code whatever the components they hold.
-template <class Point, bool TR, class Mem>
-__device__ __noinline__ int walk_fill(const Group& g, Walk& w)
+// The next chunk of intervals with steps in it; false at the end of the walk.
+__device__ __forceinline__ bool walk_chunk(const Ctx& c, int lane, Walk& w)
 {
-    constexpr int SB = Mem::SB;
-    Mem& M = group_mem<Mem>();
-    const int lane = g.lane;
+    const bool TR = w.rev;
     const bool up = w.r2 > w.r1;
     const int di = up ? 1 : -1;
     const int nint = (up ? w.i2 - w.i1 : w.i1 - w.i2) + 1;
+    const Knot* kn = c.kn;
     while (w.s0 >= w.total) {
-        if (w.r1 == w.r2 || w.q0 >= nint) return 0;
-        const Knot* kn = g.c.kn;
+        if (w.r1 == w.r2 || w.q0 >= nint) return false;
         const int q = w.q0 + lane;
         w.iv = TR ? w.i2 - di * q : w.i1 + di * q;
         w.n = 0;
@@ -405,7 +401,7 @@ __device__ __noinline__ int walk_fill(const Group& g, Walk& w)
                 rr2 = (w.iv == w.i2) ? w.r2 : kn[w.iv].r;
             }
             if (rr1 != rr2) {
-                const double nf = floor(fabs(rr2 - rr1) / steps(g.c, w.iv));
+                const double nf = floor(fabs(rr2 - rr1) / steps(c, w.iv));
                 w.n = 1 + (int)fmin(nf, 4194304.0);
                 w.x = rr1;
                 w.h = (rr2 - rr1) / (double)w.n;
@@ -422,29 +418,51 @@ __device__ __noinline__ int walk_fill(const Group& g, Walk& w)
         w.s0 = 0;
         w.q0 += 32;
     }
-    const int nb = min(SB, w.total - w.s0);
-    // point t: stage t % 6 of step t / 6 of the batch
-    const int t = (int)threadIdx.x;
-    const int sl = t / 6, st = t - 6 * sl;
-    const int s = min(w.s0 + sl, w.total - 1);
+    return true;
+}
+
+// Step s of the chunk (clamped to its last): interval, radius and size.  The
+// lanes of a warp call it together, each with its own s.
+__device__ __forceinline__ void walk_step(const Walk& w, int s, int* iv, double* x, double* h)
+{
+    s = min(s, w.total - 1);
     int L = 0;                        // intervals of the chunk that end at or before step s
 #pragma unroll
     for (int b = 16; b > 0; b >>= 1) {
         const int v = __shfl_sync(FULL, w.cum, L + b - 1);
         if (v <= s) L += b;
     }
-    const int bi = __shfl_sync(FULL, w.iv, L), bn = __shfl_sync(FULL, w.n, L);
+    const int bn = __shfl_sync(FULL, w.n, L);
     const double bx = __shfl_sync(FULL, w.x, L), bh = __shfl_sync(FULL, w.h, L);
-    const int bc = __shfl_sync(FULL, w.cum, L) - bn;
+    int j = s - (__shfl_sync(FULL, w.cum, L) - bn);
+    if (w.rev) j = bn - 1 - j;
+    *iv = __shfl_sync(FULL, w.iv, L);
+    *x = __dadd_rn(bx, __dmul_rn((double)j, bh));
+    *h = bh;
+}
+
+// The points, step sizes and intervals of the next batch of steps (yint's,
+// or in reverse order) into shared memory; returns its steps, 0 at
+// the end of the walk.  The warps of a group call it together: one copy in
+// the code whatever the components they hold.
+template <class Point, class Mem>
+__device__ __noinline__ int walk_fill(const Group& g, Walk& w)
+{
+    Mem& M = group_mem<Mem>();
+    if (!walk_chunk(g.c, g.lane, w)) return 0;
+    const int nb = min(Mem::SB, w.total - w.s0);
+    // point t: stage t % 6 of step t / 6 of the batch
+    const int t = (int)threadIdx.x;
+    const int sl = t / 6, st = t - 6 * sl;
+    int iv;
+    double x, h;
+    walk_step(w, w.s0 + sl, &iv, &x, &h);
     if (sl < nb) {
-        int j = s - bc;
-        if (TR) j = bn - 1 - j;
-        const double x = __dadd_rn(bx, __dmul_rn((double)j, bh));
         const double a = st == 0 ? 0.0 : st == 1 ? 0.2 : st == 2 ? 0.3 : st == 3 ? 0.6 : st == 4 ? 1.0 : 0.875;
-        Point::eval(g.c, bi, x + a * bh, M.pt[t]);
+        Point::eval(g.c, iv, x + a * h, M.pt[t]);
         if (st == 0) {
-            M.sh[sl] = bh;
-            M.sil[sl] = bi;
+            M.sh[sl] = h;
+            M.sil[sl] = iv;
         }
     }
     w.s0 += nb;
@@ -489,7 +507,7 @@ __device__ __noinline__ void group_walk(Group& g, int i1, int i2, double r1, dou
     const int lane = g.lane, warp = g.warp;
     const Own<NO> own = own_rows<Sys, NW, Mem>(warp);
     Walk w;
-    walk_init(w, i1, i2, r1, r2);
+    walk_init(w, i1, i2, r1, r2, TR);
     LaneCtx lc = g.lc;
     cd y[NO];
 #pragma unroll
@@ -500,7 +518,7 @@ __device__ __noinline__ void group_walk(Group& g, int i1, int i2, double r1, dou
     int scale = 0;
     long long cnt = 0;
     int nb;
-    while ((nb = walk_fill<Point, TR, Mem>(g, w)) > 0) {
+    while ((nb = walk_fill<Point, Mem>(g, w)) > 0) {
 #pragma unroll 1
         for (int s = 0; s < nb; s++) {
             if (__any_sync(FULL, !started && jl <= M.sil[s])) {       // the same lanes in every warp
