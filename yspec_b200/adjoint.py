@@ -18,7 +18,7 @@ the linear map, dL/dmm_i = <dL/dtraces, G_i> / moment_norm.
 Gradients with respect to the earth model (per-knot rho, Vp, Vs) come in
 reverse mode by default: Engine.gradient (ysg_event_gradient) carries the
 trace adjoint back through the time stage and the l-sum (their transposes)
-and through every (omega, l) solve (its discrete adjoint, k_solve_adjoint.cu)
+and through every (omega, l) solve (its discrete adjoint, k_group_adjoint.cu)
 to dL/d(knot arrays), and torch autograd takes it through the model chain
 (model_chain.KnotModel.arrays) to rho, Vp and Vs: one reverse sweep per
 pair, whatever the number of parameters.  The forward-mode alternative is

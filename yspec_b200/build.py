@@ -40,6 +40,7 @@ SOURCES = [
     CSRC / "k_solve_group.cu",
     CSRC / "k_solve_tangent.cu",
     CSRC / "k_solve_adjoint.cu",
+    CSRC / "k_group_adjoint.cu",
     CSRC / "k_schedule.cu",
     CSRC / "k_legendre.cu",
     CSRC / "k_lsum.cu",

@@ -111,6 +111,7 @@ struct ysg_handle {
     DevBuf ukn, usg;
     bool has_units = false;
     DevBuf abasis, about, ascr, acs0, agout, asbar, acoefb, agrad, alogs;
+    DevBuf agoff, agorder[2];        // item offsets and orders of the sweeps by groups
     // events
     std::vector<Slot> slots;
     int nactive = 0;                 // slots of the last prepare / batch
@@ -1134,10 +1135,11 @@ void ysg_destroy(ysg_handle* h)
     for (DevBuf* b : {&h->kn, &h->sg, &h->hdr_dev, &h->offs, &h->keys0, &h->keys1, &h->vals0,
                       &h->vals1, &h->sort_tmp, &h->poff, &h->pfx, &h->work, &h->status, &h->items, &h->counter,
                       &h->evdev, &h->coefptr, &h->tt, &h->goff, &h->gcounter, &h->dkn, &h->dsg, &h->ukn, &h->usg, &h->abasis,
-                      &h->about, &h->ascr, &h->acs0, &h->agout, &h->asbar, &h->acoefb, &h->agrad, &h->alogs})
+                      &h->about, &h->ascr, &h->acs0, &h->agout, &h->asbar, &h->acoefb, &h->agrad, &h->alogs, &h->agoff})
         b->release();
     for (DevBuf& b : h->scratch) b.release();
     for (DevBuf& b : h->gorder) b.release();
+    for (DevBuf& b : h->agorder) b.release();
     for (auto& e : h->ev)
         if (e) cudaEventDestroy(e);
     for (int i = 0; i < ysg_handle::NSIDE; i++) {
@@ -1376,7 +1378,8 @@ int ysg_event_gradient(ysg_handle* h, const ysg_event* ev, const ysg_time* tm, c
     rc = upload_event(h, s, ev);
     if (!rc) rc = upload_time(h, s, tm, ev->nw);
     if (!rc) rc = upload_batch_items(h, 1);
-    if (!rc) rc = ensure_pairs(h);
+    const bool groups = h->model_groups;
+    if (!rc && !groups) rc = ensure_pairs(h);
     if (!rc) rc = ensure_units(h);
     if (rc) return rc;
     h->nactive = 1;
@@ -1385,21 +1388,66 @@ int ysg_event_gradient(ysg_handle* h, const ysg_event* ev, const ysg_time* tm, c
     const int nout = td.nout;
     int nmax = 0, ncmax = 0, gmax = 0;
     adj_bounds(h, s.pev, &nmax, &ncmax, &gmax);
-    // sweep work space: every resident thread of the l >= 1 sweeps (step
-    // logs only) and one thread per frequency of the l = 0 sweeps (step and
-    // grid logs), within a quarter of the free memory
-    int nblk = solve_adjoint_blocks();
-    if (nblk <= 0) return YSG_ERR_CUDA;
-    size_t free_b = 0, total_b = 0;
-    CK(cudaMemGetInfo(&free_b, &total_b));
+    // sweep work space, within a quarter of the free memory: by groups, the
+    // step logs of every resident lane of the spheroidal and the toroidal
+    // sweeps, grid logs per frequency and short step logs per lane of the
+    // l = 0 sweeps; else step logs of every resident thread of the l >= 1
+    // sweeps, and step and grid logs of one thread per frequency
+    size_t budget = 0;
+    auto over = [&](size_t bytes) {               // the query is slow: only to grow the work space
+        if (bytes <= h->alogs.cap) return false;
+        if (!budget) {
+            size_t free_b = 0, total_b = 0;
+            if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return true;
+            budget = (free_b + h->alogs.cap) / 4;
+        }
+        return bytes > budget;
+    };
+    const int gkind[2] = {GROUP_SPH0 + ev->grav, GROUP_TOR};
+    long long gitems[2] = {};
+    int gblk[2] = {};
+    const size_t glane = ((size_t)nmax + ncmax) * (14 * sizeof(cd) + sizeof(double));
+    const size_t grad_b = (size_t)nw * gmax * (4 * sizeof(cd) + sizeof(double) + sizeof(int)) +
+                          (size_t)nw * 32 * adj_step_bytes(RAD_PIECE_STEPS) + 4096;
+    size_t log_bytes = 0, T = 0, Tr = 0;
+    int nblk = 0;
     const size_t per = adj_log_bytes(nmax, ncmax, 0), per_r = adj_log_bytes(nmax, ncmax, gmax);
-    const size_t Tr = ev->lmin == 0 ? (size_t)(nw + ADJ_THREADS - 1) / ADJ_THREADS * ADJ_THREADS : 0;
-    const size_t budget = (free_b + h->alogs.cap) / 4;
-    // no more threads than entries
-    nblk = (int)std::min<long long>(nblk, (2 * h->npairs + ADJ_THREADS - 1) / ADJ_THREADS);
-    while (nblk > 1 && (size_t)nblk * ADJ_THREADS * per + Tr * per_r > budget) nblk--;
-    if ((size_t)nblk * ADJ_THREADS * per + Tr * per_r > budget) return YSG_ERR_LIMIT;
-    const size_t T = (size_t)nblk * ADJ_THREADS;
+    if (groups) {
+        size_t need = ev->lmin == 0 ? grad_b : 0;
+        for (int q = 0; q < 2; q++) {
+            gitems[q] = group_items(ev->lmin, ev->lmax, nw, ev->grav, gkind[q], group_adj_width(gkind[q]));
+            if (gitems[q] >= (1ll << 31)) return YSG_ERR_LIMIT;
+            const int resident = group_adj_blocks(gkind[q]);
+            if (resident <= 0) return YSG_ERR_CUDA;
+            gblk[q] = (int)std::min<long long>(resident, gitems[q]);
+            CK(h->agorder[q].ensure(group_order_bytes(std::max<long long>(gitems[q], 1))));
+        }
+        auto total = [&]() {
+            size_t b = need;
+            for (int q = 0; q < 2; q++) b += (size_t)gblk[q] * group_adj_threads(gkind[q]) * glane;
+            return b;
+        };
+        while (over(total()) && (gblk[0] > 1 || gblk[1] > 1))
+            for (int q = 0; q < 2; q++)
+                if (gblk[q] > 1) gblk[q]--;
+        if (over(total())) return YSG_ERR_LIMIT;
+        log_bytes = total();
+        long long off[4] = {0, gitems[0], 0, gitems[1]};
+        CK(h->agoff.ensure(sizeof off));
+        CK(h->gcounter.ensure(NGROUP * sizeof(unsigned long long)));
+        CK(cudaMemcpyAsync(h->agoff.p, off, sizeof off, cudaMemcpyHostToDevice, h->st));
+        CK(cudaStreamSynchronize(h->st));
+    } else {
+        nblk = solve_adjoint_blocks();
+        if (nblk <= 0) return YSG_ERR_CUDA;
+        Tr = ev->lmin == 0 ? (size_t)(nw + ADJ_THREADS - 1) / ADJ_THREADS * ADJ_THREADS : 0;
+        // no more threads than entries
+        nblk = (int)std::min<long long>(nblk, (2 * h->npairs + ADJ_THREADS - 1) / ADJ_THREADS);
+        while (nblk > 1 && over((size_t)nblk * ADJ_THREADS * per + Tr * per_r)) nblk--;
+        if (over((size_t)nblk * ADJ_THREADS * per + Tr * per_r)) return YSG_ERR_LIMIT;
+        T = (size_t)nblk * ADJ_THREADS;
+        log_bytes = T * per + Tr * per_r;
+    }
     const size_t nspec = (size_t)nw * std::max(nr, 1);
     const size_t ngrad = (size_t)(n + 1) * NPARAM * 4;
     CK(h->abasis.ensure((size_t)2 * nw * nw * sizeof(cd)));
@@ -1410,7 +1458,7 @@ int ysg_event_gradient(ysg_handle* h, const ysg_event* ev, const ysg_time* tm, c
     CK(h->asbar.ensure(3 * nspec * sizeof(cd)));
     CK(h->acoefb.ensure((size_t)L * NCOEF * nw * sizeof(cd)));
     CK(h->agrad.ensure(ngrad * sizeof(double)));
-    CK(h->alogs.ensure(T * per + Tr * per_r));
+    CK(h->alogs.ensure(log_bytes));
     std::vector<double> cs0((size_t)4 * nw);
     for (int b = 0; b < 2 * nw; b++) {
         cs0[2 * (size_t)b] = 1.0;
@@ -1449,8 +1497,16 @@ int ysg_event_gradient(ysg_handle* h, const ysg_event* ev, const ysg_time* tm, c
         w.gi = reinterpret_cast<int*>(take((size_t)ng * nt * sizeof(int)));
         return w;
     };
-    const AdjLogs w = carve(T, ncmax, 0);
-    const AdjLogs wr = Tr ? carve(Tr, ncmax, gmax) : AdjLogs{};
+    // the states and rescaling factors alone, for the sweeps by groups
+    auto states_of = [&](size_t nt, int n) {
+        AdjStepArrays a{};
+        a.n = n;
+        a.y = reinterpret_cast<cd*>(take((size_t)n * 14 * nt * sizeof(cd)));
+        a.f = reinterpret_cast<double*>(take((size_t)n * nt * sizeof(double)));
+        return a;
+    };
+    const AdjLogs w = groups ? AdjLogs{} : carve(T, ncmax, 0);
+    const AdjLogs wr = !groups && Tr ? carve(Tr, ncmax, gmax) : AdjLogs{};
     UnitDirs u;
     for (int p = 0; p < NPARAM; p++) {
         u.kn[p] = h->ukn.as<Knot>() + (size_t)p * (n + 2);
@@ -1479,32 +1535,65 @@ int ysg_event_gradient(ysg_handle* h, const ysg_event* ev, const ysg_time* tm, c
     else
         CK(cudaMemsetAsync(h->acoefb.p, 0, (size_t)L * NCOEF * nw * sizeof(cd), h->st));
     CK(record(h, 3));
-    // the pair schedule's cost-sorted entries, then the reverse sweeps
-    StepCost sc;
-    for (int q = 0; q < NSYS_COUNT; q++) sc.flops[q] = kStepFlops[q];
-    sc.base = kPairBaseFlops;
-    unsigned long long* keys[2] = {h->keys0.as<unsigned long long>(), h->keys1.as<unsigned long long>()};
-    unsigned long long* vals[2] = {h->vals0.as<unsigned long long>(), h->vals1.as<unsigned long long>()};
-    unsigned long long* sorted = nullptr;
-    h->launches += 3;                // k_step_prefix, k_pair_cost and the sweeps (the radix sort is CUB's)
-    CK(launch_pair_schedule(h->kn.as<Knot>(), h->sg.as<Seg>(), h->hdr_dev.as<ModelHdr>(), h->evdev.as<EventDev>(),
-                            h->offs.as<long long>(), 1, h->npairs, h->poff.as<long long>(), h->nrows,
-                            h->pfx.as<int>(), sc, keys, vals, h->sort_tmp.p, h->sort_tmp.cap, &sorted, h->st));
     CK(cudaMemsetAsync(h->agrad.p, 0, ngrad * sizeof(double), h->st));
     CK(cudaMemsetAsync(h->status.p, 0, sizeof(int), h->st));
-    // the l = 0 sweeps (few, long) beside the others on a side stream
-    if (Tr) {
-        rc = fork_side(h, 1);
-        if (rc) return rc;
-        h->launches += 1;
-        CK(launch_radial_adjoint(h->kn.as<Knot>(), h->sg.as<Seg>(), h->hdr_dev.as<ModelHdr>(),
-                                 h->evdev.as<EventDev>(), u, h->acoefb.as<cd>(), wr, h->agrad.as<double>(),
-                                 h->status.as<int>(), h->side[0]));
+    if (groups) {
+        // the l = 0 sweeps (few, long chains) and the toroidal ones beside
+        // the spheroidal ones on side streams; all add to the same gradient
+        if ((rc = fork_side(h, 2))) return rc;
+        if (ev->lmin == 0) {
+            cd* gy = reinterpret_cast<cd*>(take((size_t)nw * gmax * 4 * sizeof(cd)));
+            const size_t nt = (size_t)nw * 32;
+            AdjStepArrays ws = steps_of(nt, RAD_PIECE_STEPS);
+            double* gr = reinterpret_cast<double*>(take((size_t)nw * gmax * sizeof(double)));
+            int* gi = reinterpret_cast<int*>(take((size_t)nw * gmax * sizeof(int)));
+            take(((size_t)4096 - (size_t)(base - h->alogs.as<unsigned char>()) % 4096) % 4096);
+            h->launches += 1;
+            CK(launch_group_adj_rad(h->kn.as<Knot>(), h->sg.as<Seg>(), h->hdr_dev.as<ModelHdr>(),
+                                    h->evdev.as<EventDev>(), u, h->acoefb.as<cd>(), nw, gy, gr, gi, gmax, ws,
+                                    h->agrad.as<double>(), h->status.as<int>(), h->side[1]));
+        }
+        for (int q = 0; q < 2; q++) {
+            const size_t nt = (size_t)gblk[q] * group_adj_threads(gkind[q]);
+            AdjLogs wg{};
+            wg.nthreads = (int)nt;
+            wg.s = states_of(nt, nmax);
+            wg.c = states_of(nt, ncmax);
+            int launched = 0;
+            CK(launch_group_adj(gkind[q], h->kn.as<Knot>(), h->sg.as<Seg>(), h->hdr_dev.as<ModelHdr>(),
+                                h->evdev.as<EventDev>(), u, h->acoefb.as<cd>(), h->agoff.as<long long>() + 2 * q,
+                                gitems[q], h->tt.as<double>(), h->agorder[q].p, wg, h->agrad.as<double>(),
+                                h->gcounter.as<unsigned long long>() + gkind[q], h->status.as<int>(), gblk[q],
+                                &launched, q == 0 ? h->st : h->side[0]));
+            h->launches += launched;
+        }
+        if ((rc = join_side(h, 2))) return rc;
+    } else {
+        // the pair schedule's cost-sorted entries, then the reverse sweeps
+        StepCost sc;
+        for (int q = 0; q < NSYS_COUNT; q++) sc.flops[q] = kStepFlops[q];
+        sc.base = kPairBaseFlops;
+        unsigned long long* keys[2] = {h->keys0.as<unsigned long long>(), h->keys1.as<unsigned long long>()};
+        unsigned long long* vals[2] = {h->vals0.as<unsigned long long>(), h->vals1.as<unsigned long long>()};
+        unsigned long long* sorted = nullptr;
+        h->launches += 3;                // k_step_prefix, k_pair_cost and the sweeps (the radix sort is CUB's)
+        CK(launch_pair_schedule(h->kn.as<Knot>(), h->sg.as<Seg>(), h->hdr_dev.as<ModelHdr>(), h->evdev.as<EventDev>(),
+                                h->offs.as<long long>(), 1, h->npairs, h->poff.as<long long>(), h->nrows,
+                                h->pfx.as<int>(), sc, keys, vals, h->sort_tmp.p, h->sort_tmp.cap, &sorted, h->st));
+        // the l = 0 sweeps (few, long) beside the others on a side stream
+        if (Tr) {
+            rc = fork_side(h, 1);
+            if (rc) return rc;
+            h->launches += 1;
+            CK(launch_radial_adjoint(h->kn.as<Knot>(), h->sg.as<Seg>(), h->hdr_dev.as<ModelHdr>(),
+                                     h->evdev.as<EventDev>(), u, h->acoefb.as<cd>(), wr, h->agrad.as<double>(),
+                                     h->status.as<int>(), h->side[0]));
+        }
+        CK(launch_solve_adjoint(h->kn.as<Knot>(), h->sg.as<Seg>(), h->hdr_dev.as<ModelHdr>(), h->evdev.as<EventDev>(), u,
+                                h->acoefb.as<cd>(), sorted, 2 * h->npairs, w, h->agrad.as<double>(),
+                                reinterpret_cast<unsigned long long*>(h->counter.p), h->status.as<int>(), h->st));
+        if (Tr && (rc = join_side(h, 1))) return rc;
     }
-    CK(launch_solve_adjoint(h->kn.as<Knot>(), h->sg.as<Seg>(), h->hdr_dev.as<ModelHdr>(), h->evdev.as<EventDev>(), u,
-                            h->acoefb.as<cd>(), sorted, 2 * h->npairs, w, h->agrad.as<double>(),
-                            reinterpret_cast<unsigned long long*>(h->counter.p), h->status.as<int>(), h->st));
-    if (Tr && (rc = join_side(h, 1))) return rc;
     CK(record(h, 4));
     std::vector<double> g(ngrad);
     int status = 0;

@@ -147,6 +147,30 @@ def fmt(f):
     return repr(float(f))
 
 
+REAL = {"t", "t21", "t22", "t31", "t33", "k33", "s13", "s23"}     # real in a SolidCoef
+
+
+def entry_sum(cf):
+    """(expression, common factor) of the sum of f a.c over cf."""
+    if len(cf) == 1:
+        return f"a.{cf[0][0]}", cf[0][1]
+    assert all(abs(f) == 1.0 for _, f in cf), cf
+    cf = sorted(cf, key=lambda t: t[0] in REAL)                   # complex entries first
+    sign = cf[0][1]
+    (c0, _), rest = cf[0], [(c, f * sign) for c, f in cf[1:]]
+    r = f"a.{rest[0][0]}"
+    for c, f in rest[1:]:
+        r += f" {'+' if f * rest[0][1] > 0 else '-'} a.{c}"
+    r = f"({r})" if len(rest) > 1 else r
+    return f"(a.{c0} {'+' if rest[0][1] > 0 else '-'} {r})", sign
+
+
+def fused(s, x, y, f):
+    """s + f x y as a fused complex multiply-add (cmac / cmsc of ysg_ode.cuh)."""
+    m = "cmac" if f > 0 else "cmsc"
+    return f"{m}({s}, {x}, {y})" if abs(f) == 1.0 else f"{m}({s}, {fmt(abs(f))} * {x}, {y})"
+
+
 def emit(name, n, coef_type, outs):
     fields = COEF_FIELDS[coef_type]
     L = [f"// {name}: {n} components, coefficients {coef_type}",
@@ -166,8 +190,19 @@ def emit(name, n, coef_type, outs):
         if not terms:
             L.append(f"        g[{j}] = mk(0.0);")
             continue
-        parts = [f"({fmt(f)} * a.{c}) * k[{i}]" if f != 1.0 else f"a.{c} * k[{i}]" for c, i, f in terms]
-        L.append(f"        g[{j}] = " + " + ".join(parts) + ";")
+        # entries that multiply the same component are added first
+        groups = {}
+        for c, i, f in terms:
+            groups.setdefault(i, []).append((c, f))
+        e = None
+        for i, cf in groups.items():
+            x, f = entry_sum(cf)
+            if e is None:
+                e = (f"{x} * k[{i}]" if f == 1.0 else f"-({x} * k[{i}])" if f == -1.0 else
+                     f"({fmt(f)} * {x}) * k[{i}]")
+            else:
+                e = fused(e, x, f"k[{i}]", f)
+        L.append(f"        g[{j}] = {e};")
     L.append("    }")
     L.append("    // s.e += k . (dA/da_e) y")
     L.append(f"    __device__ static __forceinline__ void cgrad(const cd* k, const cd* y, {coef_type}Bar& s)")
@@ -180,8 +215,10 @@ def emit(name, n, coef_type, outs):
         terms = by_c.get(c, [])
         if not terms:
             continue
-        parts = [f"{fmt(f)} * (k[{i}] * y[{j}])" if f != 1.0 else f"k[{i}] * y[{j}]" for i, j, f in terms]
-        L.append(f"        s.{c} += " + " + ".join(parts) + ";")
+        e = f"s.{c}"
+        for i, j, f in terms:
+            e = fused(e, f"k[{i}]", f"y[{j}]", f)
+        L.append(f"        s.{c} = {e};")
     L.append("    }")
     L.append("};")
     return "\n".join(L)

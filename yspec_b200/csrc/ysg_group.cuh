@@ -31,6 +31,7 @@
 #include "ysg_solvers.cuh"
 
 namespace ysg {
+inline namespace YSG_VARIANT {
 namespace {
 
 constexpr int PT = 20;            // doubles per point
@@ -203,7 +204,8 @@ template <int NW_, int NL_, int NMAX, int SLOTS_>
 struct GroupMem {
     static constexpr int NW = NW_, NL = NL_, SLOTS = SLOTS_;
     static constexpr int NT = 32 * NW * NL;        // threads
-    static constexpr int SB = NT / 6;   // steps per batch of points
+    static constexpr int SB = NT / 6;              // steps per batch of points
+    static constexpr bool KEEP_R = false;          // the points' radii are not kept
     static constexpr int ROWS = NMAX + (NW > 1 ? 1 : 0);   // the last row takes the empty own slots
     static constexpr int OWN = (NMAX + NW - 1) / NW;
     double pt[SB * 6][PT];                         // points of the batch
@@ -234,6 +236,8 @@ struct Group {
     int i1;                       // the lane's start level
     bool started, valid;
     long long cnt;                // steps of the valid, started lanes
+    int jq;                       // logged walks: first step of the lane in the walk it joined
+    int nlog;                     // logged walks: steps of the last one, -1 if they exceed the log
     int scale;                    // the lane's rescalings of the last walk
 };
 
@@ -460,6 +464,7 @@ __device__ __noinline__ int walk_fill(const Group& g, Walk& w)
     if (sl < nb) {
         const double a = st == 0 ? 0.0 : st == 1 ? 0.2 : st == 2 ? 0.3 : st == 3 ? 0.6 : st == 4 ? 1.0 : 0.875;
         Point::eval(g.c, iv, x + a * h, M.pt[t]);
+        if constexpr (Mem::KEEP_R) M.pr[t] = x + a * h;
         if (st == 0) {
             M.sh[sl] = h;
             M.sil[sl] = iv;
@@ -487,6 +492,17 @@ struct StageVec {
     }
 };
 
+// Log of the states before every step of a walk (and the rescaling factor
+// after it), entry (step, component) of the lanes of a launch side by side;
+// the pointers are the thread's own.
+constexpr int GLOG_N = 14;
+struct GroupLog {
+    cd* y;
+    double* f;
+    size_t stride;                // lanes of the launch
+    int cap;                      // steps
+};
+
 // yint (TR: the transposed integration, yint_T) for the whole group.  On
 // entry every warp's own components are in yio and, with more than one
 // warp, published in ex[0] (barrier passed); on exit the same holds for the
@@ -497,13 +513,16 @@ struct StageVec {
 // the third derivative the inputs of stages 5 and 6 and the result are
 // carried as partial sums, so at most four vectors are live beside the
 // derivative.
-template <class Sys, class Point, bool TR, class Mem>
-__device__ __noinline__ void group_walk(Group& g, int i1, int i2, double r1, double r2, cd* yio, const cd* start)
+template <class Sys, class Point, bool TR, class Mem, bool LOG = false>
+__device__ __noinline__ void group_walk(Group& g, int i1, int i2, double r1, double r2, cd* yio, const cd* start,
+                                        const GroupLog* lg = nullptr, int at = 0)
 {
     constexpr int NW = Mem::NW, NO = Split<Sys, NW>::NO;
     Mem& M = group_mem<Mem>();
     g.scale = 0;
+    g.nlog = 0;
     if (r2 == r1) return;
+    int lq = at;                     // log index of the next step
     const int lane = g.lane, warp = g.warp;
     const Own<NO> own = own_rows<Sys, NW, Mem>(warp);
     Walk w;
@@ -519,13 +538,19 @@ __device__ __noinline__ void group_walk(Group& g, int i1, int i2, double r1, dou
     long long cnt = 0;
     int nb;
     while ((nb = walk_fill<Point, Mem>(g, w)) > 0) {
+        if (LOG && lq + nb > lg->cap) {
+            g.nlog = -1;
+            bsync<Mem>();
+            return;
+        }
 #pragma unroll 1
-        for (int s = 0; s < nb; s++) {
+        for (int s = 0; s < nb; s++, lq++) {
             if (__any_sync(FULL, !started && jl <= M.sil[s])) {       // the same lanes in every warp
                 if (!started && jl <= M.sil[s]) {
 #pragma unroll
                     for (int k = 0; k < NO; k++) y[k] = start[k];
                     started = true;
+                    if (LOG) g.jq = lq;
                 }
                 nact = __popc(__ballot_sync(FULL, started));
                 if (NW > 1) {
@@ -535,6 +560,13 @@ __device__ __noinline__ void group_walk(Group& g, int i1, int i2, double r1, dou
             }
             // a warp none of whose lanes has started waits for the others
             if (Mem::NL > 1 && nact == 0) continue;
+            if (LOG) {
+                // streaming stores: only the reverse pass reads them back
+#pragma unroll
+                for (int k = 0; k < NO; k++)
+                    __stcs(reinterpret_cast<double2*>(lg->y + ((size_t)lq * GLOG_N + k) * lg->stride),
+                           make_double2(y[k].x, y[k].y));
+            }
             const double(*p)[PT] = M.pt + s * 6;
                             // One copy of the right-hand side in the code, the stage
             // combinations by case: six copies would overflow the
@@ -667,6 +699,7 @@ __device__ __noinline__ void group_walk(Group& g, int i1, int i2, double r1, dou
             int mx = 0;
 #pragma unroll
             for (int k = 0; k < NO; k++) mx = max(mx, max(hi_abs(y[k].x), hi_abs(y[k].y)));
+            double factor = 1.0;
             const bool small = started && mx < 0x3BC79CA1, big = started && mx > 0x4415AF1D;
             if (NW > 1 && !TR) publish(M.ex[0], own, lane, y);
             if (gany<Mem>(small || big)) {
@@ -688,6 +721,7 @@ __device__ __noinline__ void group_walk(Group& g, int i1, int i2, double r1, dou
                 const bool s1 = (sb >> lane) & 1u, b1 = (bb >> lane) & 1u;
                 if (s1 || b1) {
                     const double f = s1 ? SC_HUGE : SC_TINY;
+                    if (LOG) factor = f;
                     scale += s1 ? 1 : -1;
 #pragma unroll
                     for (int k = 0; k < NO; k++) y[k] = y[k] * f;
@@ -695,6 +729,7 @@ __device__ __noinline__ void group_walk(Group& g, int i1, int i2, double r1, dou
                 }
                 gsync<Mem>();
             }
+            if (LOG) lg->f[(size_t)lq * lg->stride] = factor;
         }
         // the points are filled again: every warp has read them.  With one
         // lane per degree the warps of a block run free between the batches,
@@ -712,6 +747,7 @@ __device__ __noinline__ void group_walk(Group& g, int i1, int i2, double r1, dou
     if (start) g.started = started;
     g.cnt += cnt;
     g.scale = scale;
+    g.nlog = lq - at;
 }
 
 // Lanes that start at or below level `last` but have not met it on a walk
@@ -734,4 +770,5 @@ __device__ __forceinline__ void group_join_rest(Group& g, int last, cd* y, const
 }
 
 }  // namespace
+}  // inline namespace
 }  // namespace ysg

@@ -68,6 +68,11 @@ cudaError_t launch_group(int kind, int form, const Knot* kn, const Seg* sg, cons
                          void* order_buf, unsigned long long* counter, unsigned long long* work, int resident,
                          int* launched, cudaStream_t st);
 
+// The items of a list longest first, in order_buf (group_order_bytes).
+cudaError_t launch_group_order(int kind, int width, const Knot* kn, const ModelHdr* mh, const EventDev* evs,
+                               const long long* off, int nev, long long nitems, const double* tt, void* order_buf,
+                               const int** order, cudaStream_t st);
+
 // Pair cost model and ordering for schedule 1 (k_schedule.cu).  off[e] is
 // the flat index of event e's first pair (off[nev] = npairs); keys and vals
 // are two pairs of npairs-element buffers; *sorted receives the buffer
@@ -159,5 +164,23 @@ cudaError_t launch_solve_adjoint(const Knot* kn, const Seg* sg, const ModelHdr* 
                                  const UnitDirs& u, const cd* coefb, const unsigned long long* pairs,
                                  long long nentries, const AdjLogs& w, double* grad,
                                  unsigned long long* counter, int* status, cudaStream_t st);
+
+// Reverse sweeps by groups of degrees (k_group_adjoint.cu), per kind a list
+// of one event's items: off = {0, nitems}; w: step logs of the launch's
+// threads (y and f are used; s for the b-vector passes and y3, c for the
+// minors and the toroidal solutions); grad and status as launch_solve_adjoint.
+int group_adj_width(int kind);
+int group_adj_threads(int kind);
+int group_adj_blocks(int kind);                   // resident grid, 0 on failure
+cudaError_t launch_group_adj(int kind, const Knot* kn, const Seg* sg, const ModelHdr* mh, const EventDev* ev,
+                             const UnitDirs& u, const cd* coefb, const long long* off, long long nitems,
+                             const double* tt, void* order_buf, const AdjLogs& w, double* grad,
+                             unsigned long long* counter, int* status, int nblk, int* launched, cudaStream_t st);
+// l = 0: grid logs of nw frequencies (gmax points each, 4 states, radius and
+// interval per point), step logs of 32 nw lanes (RAD_PIECE_STEPS entries).
+constexpr int RAD_PIECE_STEPS = 8;
+cudaError_t launch_group_adj_rad(const Knot* kn, const Seg* sg, const ModelHdr* mh, const EventDev* ev,
+                                 const UnitDirs& u, const cd* coefb, int nw, cd* gy, double* gr, int* gi, int gmax,
+                                 const AdjStepArrays& ws, double* grad, int* status, cudaStream_t st);
 
 }  // namespace ysg

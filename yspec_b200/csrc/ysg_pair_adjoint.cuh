@@ -78,12 +78,18 @@ __device__ inline void tangent_ctx(const Ctx& c, const UnitDirs& u, int p, v_tan
 // (14), 2 fluid minor (5), 3 radial with gravity (2), 4 solid minor without
 // self-gravitation (5), 5 fluid start without it (2), 6 radial without
 // gravity (2).
-template <int WHICH>
-__device__ __noinline__ void start_adj(const Ctx& c, const UnitDirs& u, int i1, double rt, const cd* yb, SegGrad& G)
+template <int WHICH, class Grad>
+__device__ __noinline__ void start_adj(const Ctx& c, const UnitDirs& u, int i1, double rt, const cd* yb, Grad& G)
 {
     constexpr int N = WHICH == 1 ? 14 : ((WHICH == 2 || WHICH == 4) ? 5 : 2);
     double vb[NPARAM];
+#pragma unroll 1
     for (int p = 0; p < NPARAM; p++) {
+        // the start vectors read rho, mu, q_mu, kappa and q_kappa only
+        if (p != P_RHO && p != P_MU && p != P_QMU && p != P_KAPPA && p != P_QKAPPA) {
+            vb[p] = 0.0;
+            continue;
+        }
         v_tangent::Ctx t;
         tangent_ctx(c, u, p, t);
         v_tangent::mcplx y[N];
@@ -104,11 +110,18 @@ __device__ __noinline__ void start_adj(const Ctx& c, const UnitDirs& u, int i1, 
 // Source vectors at (is, rs): svtb (5 x 2) and svsb (5 x 6) are the
 // adjoints of the toroidal and spheroidal source vectors (either may be
 // null).
+template <class Grad>
 __device__ __noinline__ void source_adj(const Ctx& c, const UnitDirs& u, int is, double rs, const double* mm,
-                                  const cd (*svtb)[2], const cd (*svsb)[6], SegGrad& G)
+                                  const cd (*svtb)[2], const cd (*svsb)[6], Grad& G)
 {
     double vb[NPARAM];
+#pragma unroll 1
     for (int p = 0; p < NPARAM; p++) {
+        // the source vectors read C, F, L and their attenuation only
+        if (p != P_CCON && p != P_FCON && p != P_LCON && p != P_QMU && p != P_XLAM && p != P_XA2) {
+            vb[p] = 0.0;
+            continue;
+        }
         v_tangent::Ctx t;
         tangent_ctx(c, u, p, t);
         double s = 0.0;
@@ -131,8 +144,9 @@ __device__ __noinline__ void source_adj(const Ctx& c, const UnitDirs& u, int is,
 
 // Radial source vector at (is, rs) (module_solver.f90:566-627): s0b holds
 // the adjoints of its two components.
+template <class Grad>
 __device__ __noinline__ void source_rad_adj(const Ctx& c, const UnitDirs& u, int is, double rs, const double* mm,
-                                      const cd* s0b, SegGrad& G)
+                                      const cd* s0b, Grad& G)
 {
     double vb[NPARAM];
     for (int p = 0; p < NPARAM; p++) {
@@ -931,23 +945,16 @@ __device__ inline bool pair_radial_adj(Ctx& c, const UnitDirs& u, const EventDev
     return true;
 }
 
-// wwb: adjoints of ww(1:5) of pair (l >= 2, j).  The adjoints of the
-// solver's output need only the source vectors, so the solver's reverse
-// sweep runs first and its own forward pass supplies the output that the
-// source vectors' adjoints need.
-__device__ inline bool pair_toroidal_adj(Ctx& c, const UnitDirs& u, const EventDev& ev, int l, int j,
-                                         const cd* wwb, StepLog& L, StepLog& CL, SegGrad& G)
+// Adjoints of tor_solver's output from those of ww(1:5).
+__device__ inline void toroidal_resp_adj(const Ctx& c, const EventDev& ev, int l, cd w, const cd* wwb, cd (*yb)[2])
 {
-    const cd w = omega_of(ev, j);
-    set_l(c, l);
-    set_omega(c, w);
-    cd svt[5][2], ytor[2][2];
+    cd svt[5][2];
     source_vector_tor(c, ev.is, ev.rs, ev.mm, svt);
     const cd f = out_factor(ev.out, w);
-    const double zeta = (double)sqrtf((float)(l * (l + 1)));
-    const double zr = zeta * ev.rr;
+    const double zr = (double)sqrtf((float)(l * (l + 1))) * ev.rr;
     // ww[q] = (svt[q][0] ytor'[0][0] + svt[q][1] ytor'[0][1]) / zr, ytor' = f ytor
-    cd yb[2][2] = {{mk(0.0), mk(0.0)}, {mk(0.0), mk(0.0)}};
+    for (int a = 0; a < 2; a++)
+        for (int b = 0; b < 2; b++) yb[a][b] = mk(0.0);
     for (int q = 0; q < 5; q++) {
         const cd g = wwb[q] / zr;
         yb[0][0] = yb[0][0] + g * svt[q][0];
@@ -956,7 +963,16 @@ __device__ inline bool pair_toroidal_adj(Ctx& c, const UnitDirs& u, const EventD
     if (ev.out != 0)
         for (int a = 0; a < 2; a++)
             for (int b = 0; b < 2; b++) yb[a][b] = f * yb[a][b];
-    if (!tor_solver_adj(c, u, ev.rr, ev.rs, ev.ir, ev.is, yb, ytor, L, CL, G)) return false;
+}
+
+// The rest of the toroidal epilogue, given tor_solver's output (scaled in
+// place): the source vectors' contribution.
+template <class Grad>
+__device__ inline void toroidal_rest_adj(const Ctx& c, const UnitDirs& u, const EventDev& ev, int l, cd w,
+                                         const cd* wwb, cd (*ytor)[2], Grad& G)
+{
+    const cd f = out_factor(ev.out, w);
+    const double zr = (double)sqrtf((float)(l * (l + 1))) * ev.rr;
     if (ev.out != 0)
         for (int a = 0; a < 2; a++)
             for (int b = 0; b < 2; b++) ytor[a][b] = f * ytor[a][b];
@@ -967,19 +983,31 @@ __device__ inline bool pair_toroidal_adj(Ctx& c, const UnitDirs& u, const EventD
         svtb[q][1] = g * ytor[0][1];
     }
     source_adj(c, u, ev.is, ev.rs, ev.mm, svtb, nullptr, G);
-    return true;
 }
 
-// uub, vvb: adjoints of uu(1:5), vv(1:5) of pair (l >= 1, j); the same
-// order as the toroidal part.
-__device__ inline bool pair_spheroidal_adj(Ctx& c, const UnitDirs& u, const EventDev& ev, int l, int j,
-                                           const cd* uub, const cd* vvb, StepLog& L, StepLog& CL, SegGrad& G)
+// wwb: adjoints of ww(1:5) of pair (l >= 2, j).  The adjoints of the
+// solver's output need only the source vectors, so the solver's reverse
+// sweep runs first and its own forward pass supplies the output that the
+// source vectors' adjoints need.
+__device__ inline bool pair_toroidal_adj(Ctx& c, const UnitDirs& u, const EventDev& ev, int l, int j,
+                                         const cd* wwb, StepLog& L, StepLog& CL, SegGrad& G)
 {
     const cd w = omega_of(ev, j);
     set_l(c, l);
     set_omega(c, w);
-    alpha_steps(c);
-    cd svs[5][6], ysph[6][4];
+    cd yb[2][2], ytor[2][2];
+    toroidal_resp_adj(c, ev, l, w, wwb, yb);
+    if (!tor_solver_adj(c, u, ev.rr, ev.rs, ev.ir, ev.is, yb, ytor, L, CL, G)) return false;
+    toroidal_rest_adj(c, u, ev, l, w, wwb, ytor, G);
+    return true;
+}
+
+// Adjoints of rows 0-2 of the spheroidal responses from those of uu(1:5) and
+// vv(1:5).
+__device__ inline void spheroidal_resp_adj(const Ctx& c, const EventDev& ev, int l, cd w, const cd* uub,
+                                           const cd* vvb, cd (*yb)[4])
+{
+    cd svs[5][6];
     source_vector_sph(c, ev.is, ev.rs, ev.mm, svs);
     const double zeta = (double)sqrtf((float)(l * (l + 1)));
     const cd mw2 = -(w * w);
@@ -988,8 +1016,7 @@ __device__ inline bool pair_spheroidal_adj(Ctx& c, const UnitDirs& u, const Even
     const int col[4] = {0, 1, 3, 4};
     // uu[q] = sum_b ysph'[0][b] svs[q][col b] / rr;  vv[q] = sum_b ysph'[1][b] svs[q][col b] / zr,
     // ysph' the solver output after the output scaling and corrections
-    cd yb[6][4], ybo[2][4];
-    for (int a = 0; a < 6; a++)
+    for (int a = 0; a < 3; a++)
         for (int b = 0; b < 4; b++) yb[a][b] = mk(0.0);
     for (int q = 0; q < 5; q++) {
         const cd gu = uub[q] / ev.rr, gv = vvb[q] / zr;
@@ -997,10 +1024,6 @@ __device__ inline bool pair_spheroidal_adj(Ctx& c, const UnitDirs& u, const Even
             yb[0][b] = yb[0][b] + gu * svs[q][col[b]];
             yb[1][b] = yb[1][b] + gv * svs[q][col[b]];
         }
-    }
-    for (int b = 0; b < 4; b++) {
-        ybo[0][b] = yb[0][b];
-        ybo[1][b] = yb[1][b];
     }
     // output scaling and the potential / tilt correction (yspec.f90:376-391)
     if (ev.out == 1) {
@@ -1021,31 +1044,32 @@ __device__ inline bool pair_spheroidal_adj(Ctx& c, const UnitDirs& u, const Even
             }
         }
     }
-    if (ev.grav == 2) {
-        if (!sph_solver_g_adj(c, u, ev.rr, ev.rs, ev.ir, ev.is, yb, ysph, L, CL, G)) return false;
-    } else {
-        // the 4-vector solution (U, V, R, S): its U and V rows are the
-        // outputs; the potential is zero (yspec.f90:367-374)
-        cd ybn[4][4], yng[4][4];
-        for (int b = 0; b < 4; b++) {
-            ybn[0][b] = yb[0][b];
-            ybn[1][b] = yb[1][b];
-            ybn[2][b] = ybn[3][b] = mk(0.0);
-        }
-        const bool ok = ev.grav == 1 ? sph_solver_nc_adj<1>(c, u, ev.rr, ev.rs, ev.ir, ev.is, ybn, yng, L, CL, G)
-                                     : sph_solver_nc_adj<0>(c, u, ev.rr, ev.rs, ev.ir, ev.is, ybn, yng, L, CL, G);
-        if (!ok) return false;
-        for (int b = 0; b < 4; b++) {
-            ysph[0][b] = yng[0][b];
-            ysph[1][b] = yng[1][b];
-            ysph[2][b] = mk(0.0);
-        }
-    }
+}
+
+// The rest of the spheroidal epilogue, given rows 0-2 of the responses
+// (scaled in place): the correction's and the source vectors' contributions.
+template <class Grad>
+__device__ inline void spheroidal_rest_adj(const Ctx& c, const UnitDirs& u, const EventDev& ev, int l, cd w,
+                                           const cd* uub, const cd* vvb, cd (*ysph)[4], Grad& G)
+{
+    const double zeta = (double)sqrtf((float)(l * (l + 1)));
+    const cd mw2 = -(w * w);
+    const double gr = ev.grav_ir;
+    const double zr = zeta * ev.rr;
+    const int col[4] = {0, 1, 3, 4};
     // grav(ir), the c0 coefficient of segment ir, through the correction
     if (ev.out == 2 && ev.cor != 0) {
+        cd svs[5][6];
+        source_vector_sph(c, ev.is, ev.rs, ev.mm, svs);
         double gb = 0.0;
-        for (int b = 0; b < 4; b++)
-            gb += re(ybo[0][b] * (-2.0 * ysph[0][b] / ev.rr)) + re(ybo[1][b] * (zeta * ysph[0][b] / ev.rr));
+        for (int b = 0; b < 4; b++) {
+            cd ybo[2] = {mk(0.0), mk(0.0)};       // adjoints of the corrected rows
+            for (int q = 0; q < 5; q++) {
+                ybo[0] = ybo[0] + (uub[q] / ev.rr) * svs[q][col[b]];
+                ybo[1] = ybo[1] + (vvb[q] / zr) * svs[q][col[b]];
+            }
+            gb += re(ybo[0] * (-2.0 * ysph[0][b] / ev.rr)) + re(ybo[1] * (zeta * ysph[0][b] / ev.rr));
+        }
         double vb[NPARAM];
         for (int p = 0; p < NPARAM; p++) vb[p] = 0.0;
         vb[P_GRAV] = gb;
@@ -1076,6 +1100,42 @@ __device__ inline bool pair_spheroidal_adj(Ctx& c, const UnitDirs& u, const Even
         for (int b = 0; b < 4; b++) svsb[q][col[b]] = svsb[q][col[b]] + gu * ysph[0][b] + gv * ysph[1][b];
     }
     source_adj(c, u, ev.is, ev.rs, ev.mm, nullptr, svsb, G);
+}
+
+// uub, vvb: adjoints of uu(1:5), vv(1:5) of pair (l >= 1, j); the same
+// order as the toroidal part.
+__device__ inline bool pair_spheroidal_adj(Ctx& c, const UnitDirs& u, const EventDev& ev, int l, int j,
+                                           const cd* uub, const cd* vvb, StepLog& L, StepLog& CL, SegGrad& G)
+{
+    const cd w = omega_of(ev, j);
+    set_l(c, l);
+    set_omega(c, w);
+    alpha_steps(c);
+    cd yb[6][4], ysph[6][4];
+    for (int a = 3; a < 6; a++)
+        for (int b = 0; b < 4; b++) yb[a][b] = mk(0.0);
+    spheroidal_resp_adj(c, ev, l, w, uub, vvb, yb);
+    if (ev.grav == 2) {
+        if (!sph_solver_g_adj(c, u, ev.rr, ev.rs, ev.ir, ev.is, yb, ysph, L, CL, G)) return false;
+    } else {
+        // the 4-vector solution (U, V, R, S): its U and V rows are the
+        // outputs; the potential is zero (yspec.f90:367-374)
+        cd ybn[4][4], yng[4][4];
+        for (int b = 0; b < 4; b++) {
+            ybn[0][b] = yb[0][b];
+            ybn[1][b] = yb[1][b];
+            ybn[2][b] = ybn[3][b] = mk(0.0);
+        }
+        const bool ok = ev.grav == 1 ? sph_solver_nc_adj<1>(c, u, ev.rr, ev.rs, ev.ir, ev.is, ybn, yng, L, CL, G)
+                                     : sph_solver_nc_adj<0>(c, u, ev.rr, ev.rs, ev.ir, ev.is, ybn, yng, L, CL, G);
+        if (!ok) return false;
+        for (int b = 0; b < 4; b++) {
+            ysph[0][b] = yng[0][b];
+            ysph[1][b] = yng[1][b];
+            ysph[2][b] = mk(0.0);
+        }
+    }
+    spheroidal_rest_adj(c, u, ev, l, w, uub, vvb, ysph, G);
     return true;
 }
 

@@ -12,6 +12,7 @@
 #include "ysg_group.cuh"
 
 namespace ysg {
+inline namespace YSG_VARIANT {
 namespace {
 
 // Matrix of an integration: (y0, y1) -> (a y0 + b y1, c y0 + d y1).
@@ -362,4 +363,5 @@ __device__ __noinline__ void rad_ng_warp(Ctx& c, RadMem& M, int lane, double rr,
 }
 
 }  // namespace
+}  // inline namespace
 }  // namespace ysg
