@@ -449,44 +449,26 @@ int upload_time(ysg_handle* h, Slot& s, const ysg_time* tm, int nw)
     const int nout = ysg_trace_rows(tm);
     int p = 0;
     while ((1 << p) < n) p++;
-    const double pi_d = (double)3.14159265358979323846f;
-    std::vector<double> filt((size_t)n / 2 + 1, 1.0), expt(nout), cs(2 * (size_t)std::max(nr, 1));
-    const double w1 = tm->f11, w2 = tm->f12, w3 = tm->f21, w4 = tm->f22;
-    if (!(w1 == 0.0 && w2 == 0.0 && w3 == 0.0 && w4 == 0.0)) {
-        double f = 0.0;
-        for (int i = 1; i <= n / 2 + 1; i++) {
-            double w = (double)(i - 1) * tm->df;
-            if (w < w1) f = 0.0;
-            else if (w >= w1 && w < w2) f = 0.5 * (1.0 - std::cos(pi_d * (w - w1) / (w2 - w1)));
-            else if (w >= w2 && w < w3) f = 1.0;
-            else if (w >= w3 && w < w4) f = 0.5 * (1.0 - std::cos(pi_d * (w4 - w) / (w4 - w3)));
-            else if (w >= w4) f = 0.0;
-            filt[(size_t)i - 1] = f;
-        }
-    }
-    std::vector<cd> tw((size_t)n / 2);
-    const double dth = pi_d / (double)(n / 2);     // exact: n/2 is a power of two
-    for (int m = 0; m < n / 2; m++) {
-        double a = (double)m * dth;
-        tw[(size_t)m] = mk(std::cos(a), std::sin(a));
-    }
-    for (int i = 0; i < nout; i++) expt[(size_t)i] = std::exp(tm->ep * ((double)i * tm->dt));
+    std::vector<double> cs(2 * (size_t)std::max(nr, 1));
     for (int k = 0; k < nr; k++) {
         cs[2 * (size_t)k] = std::cos(tm->azep[k]);
         cs[2 * (size_t)k + 1] = std::sin(tm->azep[k]);
     }
     s.tm_ready = false;
-    CK(s.filt.ensure(filt.size() * sizeof(double)));
-    CK(s.tw.ensure(tw.size() * sizeof(cd)));
-    CK(s.expt.ensure(expt.size() * sizeof(double)));
+    CK(s.filt.ensure(((size_t)n / 2 + 1) * sizeof(double)));
+    CK(s.tw.ensure(twiddle_count(n) * sizeof(cd)));
+    CK(s.expt.ensure((size_t)nout * sizeof(double)));
     CK(s.cs.ensure(cs.size() * sizeof(double)));
     CK(h->scratch[0].ensure(std::max<size_t>(ifft_scratch_bytes(n, nr), 16)));
     CK(s.out.ensure(std::max<size_t>((size_t)nout * 4 * nr * sizeof(double), 16)));
-    CK(cudaMemcpyAsync(s.filt.p, filt.data(), filt.size() * sizeof(double), cudaMemcpyHostToDevice, h->st));
-    CK(cudaMemcpyAsync(s.tw.p, tw.data(), tw.size() * sizeof(cd), cudaMemcpyHostToDevice, h->st));
-    CK(cudaMemcpyAsync(s.expt.p, expt.data(), expt.size() * sizeof(double), cudaMemcpyHostToDevice, h->st));
+    // the tables are formed on the device: e^{eps t} and the twiddles of a
+    // 32768-point row took 1 ms on the host
+    const bool one = n <= SERIES_MAX;
+    CK(launch_time_tables(p, one ? s.tw.as<cd>() : nullptr, n / 2, one ? nullptr : s.tw.as<cd>(),
+                          TaperDev{tm->df, tm->f11, tm->f12, tm->f21, tm->f22}, n / 2 + 1, s.filt.as<double>(), tm->ep,
+                          tm->dt, nout, s.expt.as<double>(), h->st));
     CK(cudaMemcpyAsync(s.cs.p, cs.data(), cs.size() * sizeof(double), cudaMemcpyHostToDevice, h->st));
-    h->h2d += (double)((filt.size() + expt.size() + cs.size()) * sizeof(double) + tw.size() * sizeof(cd));
+    h->h2d += (double)(cs.size() * sizeof(double));
     CK(cudaStreamSynchronize(h->st));
     TraceDev& td = s.ptd;
     td = TraceDev{};
@@ -810,7 +792,7 @@ int enqueue_traces(ysg_handle* h, int nev, int ns)
         const TraceDev& td = s.ptd;
         const size_t nspec = (size_t)td.nw * std::max(td.nr, 1);
         const cd* d_ur = s.spec.as<cd>();
-        h->launches += td.nr > 0 ? 3 : 0;   // pass A, pass B, rotation
+        h->launches += td.nr > 0 ? ifft_launches(td.nt) : 0;
         CK(launch_ifft(td, d_ur, d_ur + nspec, d_ur + 2 * nspec, s.filt.as<double>(), s.tw.as<cd>(),
                        s.expt.as<double>(), s.cs.as<double>(), h->scratch[ns ? e % ns : 0].as<cd>(),
                        s.out.as<double>(), stream_of(h, ns, e)));
@@ -835,7 +817,7 @@ int enqueue_chains(ysg_handle* h, int nev, int ns)
         const size_t nspec = (size_t)d.nw * std::max(s.nr, 1);
         cd* d_ur = s.spec.as<cd>();
         cudaStream_t st = stream_of(h, ns, e);
-        h->launches += s.nr > 0 ? 4 : 0;    // l-sum, pass A, pass B, rotation
+        h->launches += s.nr > 0 ? 1 + ifft_launches(td.nt) : 0;    // l-sum and time series
         CK(launch_lsum(d.nw, s.nr, d.lmin, d.lmax, s.coef.as<cd>(), s.leg.as<double>(), s.E.as<cd>(),
                        d_ur, d_ur + nspec, d_ur + 2 * nspec, st));
         CK(launch_ifft(td, d_ur, d_ur + nspec, d_ur + 2 * nspec, s.filt.as<double>(), s.tw.as<cd>(),
@@ -1298,13 +1280,17 @@ int ysg_model_tangent_upload(ysg_handle* h, const ysg_model* dm)
 int ysg_trace_rows(const ysg_time* tm)
 {
     if (!tm) return 0;
-    int nout = tm->nt;
-    for (int i = 1; i <= tm->nt; i++)
-        if ((double)(i - 1) * tm->dt > tm->tout) {
-            nout = i;
-            break;
-        }
-    return nout;
+    // the first i with (i - 1) dt > tout, else nt: by bisection, the times
+    // rise with i (a step that does not rise exceeds tout at once or never)
+    const auto past = [&](int i) { return (double)(i - 1) * tm->dt > tm->tout; };
+    if (tm->nt < 1 || !past(tm->nt)) return tm->nt >= 1 && past(1) ? 1 : tm->nt;
+    int lo = 0, hi = tm->nt;         // past(hi), not past(lo)
+    while (hi - lo > 1) {
+        const int mid = lo + (hi - lo) / 2;
+        if (past(mid)) hi = mid;
+        else lo = mid;
+    }
+    return hi;
 }
 
 int ysg_event_coef(ysg_handle* h, const ysg_event* ev, double* coef)
@@ -1521,7 +1507,7 @@ int ysg_event_gradient(ysg_handle* h, const ysg_event* ev, const ysg_time* tm, c
     }
     CK(record(h, 1));
     // time stage on the basis, then its transpose and the l-sum's
-    h->launches += nr > 0 ? 6 : 0;   // basis, pass A, pass B, rotation, spectrum and l-sum transposes
+    h->launches += nr > 0 ? 3 + ifft_launches(td.nt) : 0;   // basis and its time series, spectrum and l-sum transposes
     if (nr > 0) {
         CK(launch_time_basis(td, h->abasis.as<cd>(), s.filt.as<double>(), s.tw.as<cd>(), s.expt.as<double>(),
                              h->acs0.as<double>(), h->ascr.as<cd>(), h->about.as<double>(), h->st));

@@ -106,7 +106,25 @@ struct TraceDev {
     int nt, i1, i2, nw, nr, nout, log2n, b1;
     double dt, scale, t_norm, amp_norm;
 };
-size_t ifft_scratch_bytes(int nt, int nr);
+struct TaperDev {
+    double df, w1, w2, w3, w4;
+};
+// Longest row of the one-kernel transform; tw below holds the twiddles of
+// every stage up to there, those of the last stage beyond (k_time_tables).
+constexpr int SERIES_MAX = 65536;
+inline size_t twiddle_count(int nt) { return nt <= SERIES_MAX ? (size_t)nt - 1 : (size_t)nt / 2; }
+inline int ifft_launches(int nt) { return nt <= SERIES_MAX ? 1 : 3; }
+cudaError_t launch_time_tables(int nstage, cd* tws, int nhalf, cd* tw, const TaperDev& f, int nbin, double* filt,
+                               double ep, double dt, int nout, double* expt, cudaStream_t st);
+cudaError_t launch_series(const TraceDev& td, const cd* ur, const cd* ut, const cd* up, const double* filt,
+                          const cd* tws, const double* expt, const double* cs, const double* azep, double* out,
+                          cudaStream_t st);
+cudaError_t launch_ifft_a(const TraceDev& td, const cd* ur, const cd* ut, const cd* up, const double* filt,
+                          const cd* tw, cd* scratch, cudaStream_t s);
+cudaError_t launch_ifft_b(const TraceDev& td, const cd* tw, const double* expt, const cd* scratch, double* out,
+                          cudaStream_t s);
+cudaError_t launch_ifft_rotate(const TraceDev& td, const double* cs, const double* azep, double* out, cudaStream_t s);
+size_t ifft_scratch_bytes(int nt, int nr);        // 0 up to SERIES_MAX
 cudaError_t launch_ifft(const TraceDev& td, const cd* ur, const cd* ut, const cd* up,
                         const double* filt, const cd* tw, const double* expt,
                         const double* cs_azep, cd* scratch, double* out, cudaStream_t s);
