@@ -77,6 +77,10 @@ void ysh_model_view(const ysh_model *m, ysg_model *view);
 int ysh_model_nknot(const ysh_model *m);
 const double *ysh_model_array(const ysh_model *m, const char *name);
 void ysh_free_model(ysh_model *m);
+/* Natural-spline second derivatives (module_spline.f90:40-73, layers split at
+ * repeated radii) of m arrays at the knots x[0..n-1]: y and y2 are n x m, the
+ * values of one knot side by side. */
+int ysh_spline_arrays(int n, const double *x, int m, const double *y, double *y2);
 /* Normalise the inputs, fcal, radius indices, geometry: yspec.f90:144-215.
  * Allocates e->delta/azst/azep (free with ysh_free_event). */
 int ysh_event_setup(const ysh_model *m, const ysh_params *p, ysh_event *e);

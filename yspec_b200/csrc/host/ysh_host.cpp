@@ -126,6 +126,37 @@ void natural_spline(const double* x, const double* y, int n, double* y2)
     for (int j = n - 2; j >= 0; j--) y2[j] = y2[j] - gam[j + 1] * y2[j + 1];
 }
 
+// The same for m arrays side by side (y and y2: n x m), one layer.
+void natural_splines(const double* x, const double* y, int n, int m, double* y2)
+{
+    const size_t M = (size_t)m;
+    if (n < 2) {
+        for (size_t k = 0; k < (size_t)n * M; k++) y2[k] = 0.0;
+        return;
+    }
+    std::vector<double> h(n, 0.0), gam(n, 0.0);
+    for (int i = 0; i + 1 < n; i++) h[i] = x[i + 1] - x[i];
+    double bet = 1.0;
+    for (size_t k = 0; k < M; k++) y2[k] = 0.0 / bet;
+    for (int j = 1; j < n; j++) {
+        const bool end = j == n - 1;
+        const double sub = end ? 0.0 : h[j - 1];
+        gam[j] = (j == 1 ? 0.0 : h[j - 1]) / bet;
+        bet = (end ? 1.0 : 2.0 * (h[j] + sub)) - sub * gam[j];
+        const double *a = y + (size_t)(j - 1) * M, *b = a + M, *c = end ? b : b + M, *up = y2 + (size_t)(j - 1) * M;
+        double* u = y2 + (size_t)j * M;
+        const double hl = h[j - 1], hr = h[j];
+        for (size_t k = 0; k < M; k++) {
+            const double rhs = end ? 0.0 : 6.0 * ((c[k] - b[k]) / hr) - 6.0 * ((b[k] - a[k]) / hl);
+            u[k] = (rhs - sub * up[k]) / bet;
+        }
+    }
+    for (int j = n - 2; j >= 0; j--) {
+        double* u = y2 + (size_t)j * M;
+        for (size_t k = 0; k < M; k++) u[k] = u[k] - gam[j + 1] * u[k + M];
+    }
+}
+
 // Cubic spline value on interval [lo, lo+1] (module_spline.f90:262-283).
 double spline_eval(const std::vector<double>& xa, const std::vector<double>& ya,
                    const std::vector<double>& y2, double x, int lo)
@@ -383,6 +414,22 @@ void ysh_model_view(const ysh_model* m, ysg_model* v)
 }
 
 int ysh_model_nknot(const ysh_model* m) { return m->nknot; }
+
+int ysh_spline_arrays(int n, const double* x, int m, const double* y, double* y2)
+{
+    if (n < 1 || m < 0 || !x || (m > 0 && (!y || !y2))) return YSG_ERR_ARG;
+    try {
+        for (int lo = 0; lo < n;) {
+            int hi = lo;
+            while (hi + 1 < n && x[hi + 1] != x[hi]) hi++;
+            natural_splines(x + lo, y + (size_t)lo * m, hi - lo + 1, m, y2 + (size_t)lo * m);
+            lo = hi + 1;
+        }
+    } catch (const std::bad_alloc&) {
+        return YSG_ERR_LIMIT;
+    }
+    return YSG_OK;
+}
 
 const double* ysh_model_array(const ysh_model* m, const char* name)
 {

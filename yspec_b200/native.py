@@ -83,7 +83,7 @@ EXPORTS = [
     "ysg_last_timings", "ysg_last_work", "ysg_last_bytes", "ysg_last_launches", "ysg_fp64_peak", "ysg_status_string",
     "ysg_last_cuda_error", "ysg_destroy", "ysg_traces_noalloc",
     "ysh_norms_get", "ysh_read_params", "ysh_free_params", "ysh_read_model", "ysh_model_view",
-    "ysh_model_nknot", "ysh_model_array", "ysh_free_model", "ysh_event_setup", "ysh_free_event",
+    "ysh_model_nknot", "ysh_model_array", "ysh_spline_arrays", "ysh_free_model", "ysh_event_setup", "ysh_free_event",
     "ysh_write_traces", "ysh_format_e15_6", "ysh_run", "ysh_run_batch", "ysh_run_potential",
     "ysh_write_potential", "ysh_free", "ysh_status_string",
 ]
@@ -154,6 +154,7 @@ def lib() -> C.CDLL:
     L.ysh_model_nknot.argtypes = [vp]
     L.ysh_model_array.argtypes = [vp, C.c_char_p]
     L.ysh_model_array.restype = _dp
+    L.ysh_spline_arrays.argtypes = [C.c_int, _dp, C.c_int, _dp, _dp]
     L.ysh_free_model.argtypes = [vp]
     L.ysh_free_model.restype = None
     L.ysh_event_setup.argtypes = [vp, C.POINTER(YshParams), C.POINTER(YshEvent)]
