@@ -273,7 +273,9 @@ int ysg_last_schedule(ysg_handle *h, int *sched, float tune_ms[3]);
 int ysg_last_timings(ysg_handle *h, float ms[4]);
 
 /* Counters of the last solve stage: number of (omega,l) pairs and the
- * algorithmic FP64 flop count of the stepping work actually performed. */
+ * algorithmic FP64 flop count of the stepping work actually performed (solves
+ * that events of a batch share, those that differ in the moment tensor
+ * alone, count once). */
 int ysg_last_work(ysg_handle *h, double *pairs, double *flops);
 
 /* Kernels of this library enqueued since the last ysg_event_prepare (or

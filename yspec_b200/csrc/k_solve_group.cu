@@ -114,21 +114,6 @@ __device__ __noinline__ void sph_resp(int lane, const cd* mb, cd delta, double f
     y4[2] = ((-u[3]) / delta) * f;
     y4[3] = ((-u[4]) / delta) * f;
 }
-__device__ __noinline__ void sph_store(const Group& g, const EventDev& ev, int j, cd (*ysph)[4], cd* coef)
-{
-    cd uu[5], vv[5];
-    const int l = g.c.ll;
-    spheroidal_coefs(g.c, ev, l, g.c.omega, ysph, uu, vv);
-    if (!g.valid) return;
-    cd* dst = coef + (size_t)(l - ev.lmin) * NCOEF * ev.nw + (j - 1);
-    // streaming stores: not read again in this launch
-    for (int q = 0; q < 5; q++) {
-        __stcs(reinterpret_cast<double2*>(dst + (size_t)q * ev.nw), make_double2(uu[q].x, uu[q].y));
-        __stcs(reinterpret_cast<double2*>(dst + (size_t)(q + 5) * ev.nw), make_double2(vv[q].x, vv[q].y));
-        if (l < 2) __stcs(reinterpret_cast<double2*>(dst + (size_t)(q + 10) * ev.nw), make_double2(0.0, 0.0));
-    }
-}
-
 struct GroupArgs {
     const Knot* kn;
     const Seg* sg;
@@ -141,7 +126,31 @@ struct GroupArgs {
     long long nitems;
     unsigned long long* counter;
     unsigned long long* work;
+    const int* next;              // per event the next one with the same solves, or -1; null: none
 };
+
+// The coefficients of the item's event, and of the events of the batch that
+// differ from it in the moment tensor alone (a.next): they have the same
+// responses.
+__device__ __noinline__ void sph_store(const Group& g, const GroupArgs& a, const Item& w, const cd (*ysph)[4])
+{
+    const int l = g.c.ll;
+    for (int e = w.e; e >= 0; e = a.next ? a.next[e] : -1) {
+        const EventDev& ev = a.evs[e];
+        cd y[3][4], uu[5], vv[5];                     // the responses are scaled in place
+        for (int k = 0; k < 3; k++)
+            for (int i = 0; i < 4; i++) y[k][i] = ysph[k][i];
+        spheroidal_coefs(g.c, ev, l, g.c.omega, y, uu, vv);
+        if (!g.valid) continue;
+        cd* dst = a.coefs[e] + (size_t)(l - ev.lmin) * NCOEF * ev.nw + (w.j - 1);
+        // streaming stores: not read again in this launch
+        for (int q = 0; q < 5; q++) {
+            __stcs(reinterpret_cast<double2*>(dst + (size_t)q * ev.nw), make_double2(uu[q].x, uu[q].y));
+            __stcs(reinterpret_cast<double2*>(dst + (size_t)(q + 5) * ev.nw), make_double2(vv[q].x, vv[q].y));
+            if (l < 2) __stcs(reinterpret_cast<double2*>(dst + (size_t)(q + 10) * ev.nw), make_double2(0.0, 0.0));
+        }
+    }
+}
 
 __device__ __forceinline__ void group_ctx(Group& g, const GroupArgs& a)
 {
@@ -344,7 +353,7 @@ __global__ void __launch_bounds__(32 * NW, MINB) k_group_split(GroupArgs a)
             if (serial) sph_resp<NW>(lane, mb, delta, huge_pow(scale3 - g.scale), ysph[k]);
         }
         count_work(g, a.work, BT::CLS);
-        if (serial) sph_store(g, ev, w.j, ysph, a.coefs[w.e]);
+        if (serial) sph_store(g, a, w, ysph);
         __syncthreads();
     }
 }
@@ -439,7 +448,7 @@ __global__ void __launch_bounds__(32 * NL, MINB) k_group_lane(GroupArgs a)
             S::resp(mb, ms3, up, delta, huge_pow(scale3 - g.scale), ysph[k]);
         }
         count_work(g, a.work, Bvec::CLS);
-        sph_store(g, ev, w.j, ysph, a.coefs[w.e]);
+        sph_store(g, a, w, ysph);
         bsync<Mem>();
     }
 }
@@ -466,10 +475,8 @@ __global__ void __launch_bounds__(32 * NL, MINB) k_group_tor(GroupArgs a)
         const EventDev& ev = a.evs[w.e];
         item_ctx(g, ev, w, (int)threadIdx.x);
         const int l = g.c.ll;
-        cd ww[5];
-        if (ev.pot) {                                 // toroidal motion carries no potential
-            for (int q = 0; q < 5; q++) ww[q] = mk(0.0);
-        } else {
+        cd yt[2][2];
+        if (!ev.pot) {                                // toroidal motion carries no potential
             const ModelHdr* mh = g.c.mh;
             const Knot* kn = g.c.kn;
             const double rr = ev.rr, rs = ev.rs;
@@ -485,7 +492,7 @@ __global__ void __launch_bounds__(32 * NL, MINB) k_group_tor(GroupArgs a)
             g.started = false;
             double rmin;
             const int imin = block_min<Mem>(g, g.i1, kn[i1].r, &rmin);
-            cd y1[2], y2[2], y3[2], yt[2][2];
+            cd y1[2], y2[2], y3[2];
             y1[0] = y1[1] = mk(0.0);
             group_walk<TorSys, TorPoint, false, Mem>(g, imin, top, rmin, up ? rs : rr, y1, s);
             group_join_rest<TorSys, Mem>(g, top, y1, s);
@@ -517,12 +524,18 @@ __global__ void __launch_bounds__(32 * NL, MINB) k_group_tor(GroupArgs a)
                     for (int q = 0; q < 2; q++) yt[p][q] = yt[p][q] * f;
             }
             count_work(g, a.work, TorSys::CLS);
-            toroidal_coefs(g.c, ev, l, g.c.omega, yt, ww);
         }
-        if (g.valid) {
-            cd* dst = a.coefs[w.e] + ((size_t)(l - ev.lmin) * NCOEF + 10) * ev.nw + (w.j - 1);
+        for (int e = w.e; e >= 0; e = a.next ? a.next[e] : -1) {       // as sph_store
+            const EventDev& em = a.evs[e];
+            cd ww[5] = {mk(0.0), mk(0.0), mk(0.0), mk(0.0), mk(0.0)};
+            if (!em.pot) {
+                cd y[2][2] = {{yt[0][0], yt[0][1]}, {yt[1][0], yt[1][1]}};
+                toroidal_coefs(g.c, em, l, g.c.omega, y, ww);
+            }
+            if (!g.valid) continue;
+            cd* dst = a.coefs[e] + ((size_t)(l - em.lmin) * NCOEF + 10) * em.nw + (w.j - 1);
             for (int q = 0; q < 5; q++)
-                __stcs(reinterpret_cast<double2*>(dst + (size_t)q * ev.nw), make_double2(ww[q].x, ww[q].y));
+                __stcs(reinterpret_cast<double2*>(dst + (size_t)q * em.nw), make_double2(ww[q].x, ww[q].y));
         }
         bsync<Mem>();
     }
@@ -557,17 +570,20 @@ __global__ void __launch_bounds__(32) k_group_rad(GroupArgs a)
     alpha_steps(c);
     cd sr0[2], yrad[2][2], ph[2] = {mk(0.0), mk(0.0)};
     unsigned n = 0;
-    source_vector_rad(c, ev.is, ev.rs, ev.mm, sr0);
     if (ev.grav != 0) rad_wg_warp(c, M, lane, ev.rr, ev.rs, yrad, ev.pot ? ph : nullptr, &n);
     else if (!ev.pot) rad_ng_warp(c, M, lane, ev.rr, ev.rs, ev.ir, ev.is, yrad, &n);
-    cd u3;
-    if (ev.pot) u3 = (sr0[0] * ph[0] + sr0[1] * ph[1]) / ev.rr;     // no gravity, no potential
-    else u3 = (sr0[0] * yrad[0][0] + sr0[1] * yrad[0][1]) / ev.rr;
-    if (ev.out != 0) u3 = out_factor(ev.out, c.omega) * u3;
-    cd* dst = a.coefs[lo] + (j - 1);
-    if (lane < NCOEF)
-        __stcs(reinterpret_cast<double2*>(dst + (size_t)lane * ev.nw),
-               lane == 2 ? make_double2(u3.x, u3.y) : make_double2(0.0, 0.0));
+    for (int e = lo; e >= 0; e = a.next ? a.next[e] : -1) {            // as sph_store
+        const EventDev& em = a.evs[e];
+        source_vector_rad(c, em.is, em.rs, em.mm, sr0);
+        cd u3;
+        if (em.pot) u3 = (sr0[0] * ph[0] + sr0[1] * ph[1]) / em.rr;    // no gravity, no potential
+        else u3 = (sr0[0] * yrad[0][0] + sr0[1] * yrad[0][1]) / em.rr;
+        if (em.out != 0) u3 = out_factor(em.out, c.omega) * u3;
+        cd* dst = a.coefs[e] + (j - 1);
+        if (lane < NCOEF)
+            __stcs(reinterpret_cast<double2*>(dst + (size_t)lane * em.nw),
+                   lane == 2 ? make_double2(u3.x, u3.y) : make_double2(0.0, 0.0));
+    }
     n = __reduce_add_sync(FULL, n);
     if (lane == 0 && n) atomicAdd(&a.work[RadSys::CLS], (unsigned long long)n);
 }
@@ -717,12 +733,12 @@ cudaError_t launch_group_order(int kind, int width, const Knot* kn, const ModelH
 cudaError_t launch_group(int kind, int form, const Knot* kn, const Seg* sg, const ModelHdr* mh, const EventDev* evs,
                          cd* const* coefs, const long long* off, int nev, long long nitems, const double* tt,
                          void* order_buf, unsigned long long* counter, unsigned long long* work, int resident,
-                         int* launched, cudaStream_t st)
+                         const int* next, int* launched, cudaStream_t st)
 {
     *launched = 0;
     if (nitems <= 0) return cudaSuccess;
     if (nitems >= (1ll << 31)) return cudaErrorInvalidValue;
-    GroupArgs a{kn, sg, mh, evs, coefs, off, nullptr, nev, nitems, counter, work};
+    GroupArgs a{kn, sg, mh, evs, coefs, off, nullptr, nev, nitems, counter, work, next};
     const GroupKernel k = group_kernel(kind, form);
     if (kind == GROUP_RAD) {
         k_group_rad<<<(unsigned)nitems, 32, 0, st>>>(a);

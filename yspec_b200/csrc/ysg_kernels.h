@@ -66,7 +66,7 @@ size_t group_order_bytes(long long nitems);
 cudaError_t launch_group(int kind, int form, const Knot* kn, const Seg* sg, const ModelHdr* mh, const EventDev* evs,
                          cd* const* coefs, const long long* off, int nev, long long nitems, const double* tt,
                          void* order_buf, unsigned long long* counter, unsigned long long* work, int resident,
-                         int* launched, cudaStream_t st);
+                         const int* next, int* launched, cudaStream_t st);
 
 // The items of a list longest first, in order_buf (group_order_bytes).
 cudaError_t launch_group_order(int kind, int width, const Knot* kn, const ModelHdr* mh, const EventDev* evs,
