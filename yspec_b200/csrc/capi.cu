@@ -364,19 +364,29 @@ int upload_items(ysg_handle* h, const std::vector<EventDev>& evs, const std::vec
     }
     for (int k = 0; k < NGROUP && h->groups; k++) {
         long long* o = &goff[(size_t)k * (evs.size() + 1)];
-        // The wide form where its items fill the GPU twice, else the narrow
-        // one: with 1.0 items per resident block (31,003 pairs) the wide
-        // form took 2.5 ms and the narrow one 1.85 ms, with 4.3 (300,000
-        // pairs) 11.6 and 16.2 ms.
+        long long n[NGROUP_FORM];
         for (int form = 0; form < NGROUP_FORM; form++) {
             if (h->gblocks[k][form] == 0) h->gblocks[k][form] = group_blocks(k, form);
             if (h->gblocks[k][form] == 0) return YSG_ERR_CUDA;
-            const int width = group_form_width(k, form);
+            n[form] = 0;
             for (size_t e = 0; e < evs.size(); e++)
-                o[e + 1] = o[e] + (lead[e] ? group_items(evs[e].lmin, evs[e].lmax, evs[e].nw, evs[e].grav, k, width) : 0);
-            h->gform[k] = form;
-            if (o[evs.size()] >= 2 * (long long)h->gblocks[k][form]) break;
+                if (lead[e])
+                    n[form] += group_items(evs[e].lmin, evs[e].lmax, evs[e].nw, evs[e].grav, k, group_form_width(k, form));
         }
+        // The wide form where its items fill the GPU twice (three times
+        // without self-gravitation) and their lanes, else the narrow one.
+        // With 1.0 items per resident block (31,003 pairs) the wide form took
+        // 2.5 ms and the narrow one 1.85 ms, with 4.3 (300,000 pairs) 11.6
+        // and 16.2 ms: with full lanes the narrow one takes 1.4 times as long,
+        // so that it pays where under 2.9 of its items make one wide one (4
+        // do with full lanes): a batch of 24 events of up to 72 degrees went
+        // from 6.8 to 5.4 ms with that part of the rule.
+        const long long fill = (k == GROUP_SPH0 || k == GROUP_SPH1 ? 3 : 2) * (long long)h->gblocks[k][0];
+        const int form = n[0] >= fill && 10 * n[1] >= 29 * n[0] ? 0 : 1;
+        for (size_t e = 0; e < evs.size(); e++)
+            o[e + 1] = o[e] + (lead[e] ? group_items(evs[e].lmin, evs[e].lmax, evs[e].nw, evs[e].grav, k,
+                                                     group_form_width(k, form)) : 0);
+        h->gform[k] = form;
         h->gitems[k] = o[evs.size()];
         h->groups = h->groups && h->gitems[k] < (1ll << 31);
     }
@@ -496,8 +506,8 @@ int upload_time(ysg_handle* h, Slot& s, const ysg_time* tm, int nw)
     CK(s.cs.ensure(cs.size() * sizeof(double)));
     CK(h->scratch[0].ensure(std::max<size_t>(ifft_scratch_bytes(n, nr), 16)));
     CK(s.out.ensure(std::max<size_t>((size_t)nout * 4 * nr * sizeof(double), 16)));
-    // the tables are formed on the device: e^{eps t} and the twiddles of a
-    // 32768-point row took 1 ms on the host
+    // formed on the device: n / 2 sines and cosines and nout exponentials
+    // per prepared event were host loops and uploads
     const bool one = n <= SERIES_MAX;
     CK(launch_time_tables(p, one ? s.tw.as<cd>() : nullptr, n / 2, one ? nullptr : s.tw.as<cd>(),
                           TaperDev{tm->df, tm->f11, tm->f12, tm->f21, tm->f22}, n / 2 + 1, s.filt.as<double>(), tm->ep,

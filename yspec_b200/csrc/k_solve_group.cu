@@ -662,6 +662,10 @@ struct GroupKernel {
     int width;                    // degrees per item
 };
 // The forms of a kind's kernel: 0 for lists that fill the GPU, 1 for short ones.
+// The kernels without self-gravitation take 255 registers (eight warps per
+// SM) too: with 168 their stepping loops spilled 50 values.  Short lists:
+// 0.73 -> 0.55 ms (41 degrees to 6 mHz), 1.33 -> 1.0 ms (Cowling,
+// 295 degrees to 20 mHz); long ones: 600 degrees to 43 mHz 3.75 -> 3.16 ms.
 GroupKernel group_kernel(int kind, int form)
 {
     switch (kind) {
@@ -669,11 +673,11 @@ GroupKernel group_kernel(int kind, int form)
             if (form == 0) return {k_group_lane<2, 4, 2>, 128, sizeof(LaneMem<2, 4>), 128};
             return {k_group_split<2, 4>, 64, sizeof(SphMemOf<2>), 32};
         case GROUP_SPH1:
-            if (form == 0) return {k_group_lane<1, 4, 3>, 128, sizeof(LaneMem<1, 4>), 128};
-            return {k_group_lane<1, 1, 12>, 32, sizeof(LaneMem<1, 1>), 32};
+            if (form == 0) return {k_group_lane<1, 4, 2>, 128, sizeof(LaneMem<1, 4>), 128};
+            return {k_group_lane<1, 1, 8>, 32, sizeof(LaneMem<1, 1>), 32};
         case GROUP_SPH0:
-            if (form == 0) return {k_group_lane<0, 4, 3>, 128, sizeof(LaneMem<0, 4>), 128};
-            return {k_group_lane<0, 1, 12>, 32, sizeof(LaneMem<0, 1>), 32};
+            if (form == 0) return {k_group_lane<0, 4, 2>, 128, sizeof(LaneMem<0, 4>), 128};
+            return {k_group_lane<0, 1, 8>, 32, sizeof(LaneMem<0, 1>), 32};
         case GROUP_TOR:
             if (form == 0) return {k_group_tor<4, 4>, 128, sizeof(TorMem<4>), 128};
             return {k_group_tor<1, 16>, 32, sizeof(TorMem<1>), 32};
