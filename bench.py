@@ -544,13 +544,13 @@ def run_b200(args) -> None:
                     "d2h_bytes_per_step": int(d2h), "ms_per_step": e_ms / args.steps},
             "gpu_launches": launches,
             "roofline": {"bound": "fp64", "pipe": "FP64 CUDA-core FMA pipe (the radial solves use no tensor cores)",
-                         "kernel": "k_solve_batched" if args.solver == "batched" else "k_solve_plain",
+                         "kernel": "k_group_lane" if args.solver == "batched" else "k_solve_plain",
                          "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                          "frac": achieved / peak if peak else None,
                          "peak_source": "measured: FP64 FMA microbenchmark run by this bench on this GPU",
                          "flops_per_launch": flops, "launch_ms": mean_solve,
                          "traffic": traffic_from_profiles(
-                             "k_solve_batched" if args.solver == "batched" else "k_solve_plain")},
+                             "k_group_lane" if args.solver == "batched" else "k_solve_plain")},
             "clocks": clk,
         }
         st = dict(zip(["legendre", "solve", "lsum", "ifft"], eng.timings()))
@@ -564,7 +564,7 @@ def run_b200(args) -> None:
                      "achieved_tflops": lsum_flops / (st["lsum"] / 1e3) / 1e12,
                      "frac_of_fp64_peak": lsum_flops / (st["lsum"] / 1e3) / 1e12 / peak,
                      "flops": lsum_flops},
-            "ifft": {"kernels": "k_ifft_a2, k_ifft_b2, k_rotate",
+            "ifft": {"kernels": "k_series",
                      "achieved_gbs": ifft_bytes / (st["ifft"] / 1e3) / 1e9,
                      "frac_of_hbm": ifft_bytes / (st["ifft"] / 1e3) / 1e9 / hbm["hbm_gbs"],
                      "hbm_peak_gbs": hbm["hbm_gbs"], "hbm_peak_source": hbm["source"],

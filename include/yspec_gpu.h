@@ -200,8 +200,9 @@ int ysg_get_stream(ysg_handle *h, void **stream);
  * (nw, nr) device arrays, d_azep has nr entries, d_out receives
  * (nout, 4, nr); tm->azep is not used.  Work is enqueued on `stream`
  * (a cudaStream_t, or NULL) and the call returns without waiting.
- * Intermediate rows live in one 16 MiB array compiled into the library and
- * held by every GPU that loads it until exit; nt is limited to 262144
+ * The call's tables, and rows beyond nt = 65536, live in one 16 MiB array
+ * compiled into the library and held by every GPU that loads it until exit;
+ * nt is limited to 262144
  * (YSG_ERR_LIMIT beyond).  All calls share that array: calls that overlap
  * on the GPU race and must be serialised.  The first call on each device
  * looks up the array's device address and should come before any stream
