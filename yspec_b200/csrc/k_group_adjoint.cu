@@ -121,7 +121,7 @@ struct SolidPointAdj {
 
 template <int KIND>
 struct FluidPointAdj {
-    using Point = FluidPoint;
+    using Point = FluidPoint<KIND>;
     using Bar = FluidCoefBar;
     static constexpr int NV = 7;
     __device__ static __forceinline__ FluidCoef amat(const LaneCtx& c) { return fluid_amat<KIND>(c, 0.0); }
@@ -703,7 +703,7 @@ __global__ void __launch_bounds__(32 * NL, MINB) k_gadj_sph(AdjArgs a)
                 } else if (ic) {
                     S::to_fluid(ms1, mf);
                 }
-                group_walk<Fluid, FluidPoint, false, Mem, true>(g, q.i1, q.i2, q.r1, q.r2, mf, leg == 1 ? st : nullptr,
+                group_walk<Fluid, FluidPoint<KIND>, false, Mem, true>(g, q.i1, q.i2, q.r1, q.r2, mf, leg == 1 ? st : nullptr,
                                                                &chain, at[leg]);
             } else {
                 if (leg == 4 && !mh->ocean)

@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(32 * NW, MINB) k_group_split(GroupArgs a)
                     if (leg == 3) sph_unit<MF, NW>(g, yf);
                     sph_publish<MF, NW>(g, yf);
                 }
-                group_walk<MF, FluidPoint, false, SphMem>(g, q.i1, q.i2, q.r1, q.r2, yf, leg == 1 ? s5 : nullptr);
+                group_walk<MF, FluidPoint<2>, false, SphMem>(g, q.i1, q.i2, q.r1, q.r2, yf, leg == 1 ? s5 : nullptr);
                 if (leg == 1) group_join_rest<MF, SphMem>(g, noc, yf, s5);
                 count_work(g, a.work, MF::CLS);
                 if (serial) sph_f2s<NW>(lane);
@@ -415,7 +415,7 @@ __global__ void __launch_bounds__(32 * NL, MINB) k_group_lane(GroupArgs a)
                 } else if (ic) {
                     S::to_fluid(ms1, mf);
                 }
-                group_walk<Fluid, FluidPoint, false, Mem>(g, q.i1, q.i2, q.r1, q.r2, mf, leg == 1 ? st : nullptr);
+                group_walk<Fluid, FluidPoint<KIND>, false, Mem>(g, q.i1, q.i2, q.r1, q.r2, mf, leg == 1 ? st : nullptr);
                 if (leg == 1) group_join_rest<Fluid, Mem>(g, noc, mf, st);
                 count_work(g, a.work, Fluid::CLS);
                 S::to_solid(mf, leg == 1 ? ms1 : ms2);

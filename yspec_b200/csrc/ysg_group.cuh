@@ -85,21 +85,30 @@ struct SolidPoint {
     }
 };
 
-// cccon | omega^-2 ri^2 | -omega^2 rho - 4 rho g ri | ri, rho | g, 1/rho
+// cccon | omega^-2 ri^2 | -omega^2 rho (- 4 rho g ri with gravity) | ri, rho | g (0 without), 1/rho.
+// Without gravity no gravity term enters the third number: adding it here and
+// taking it out per lane would lose the digits it is larger by (at 0.1 mHz
+// some 30 times omega^2 rho).
+template <int KIND>
 struct FluidPoint {
     __device__ static __forceinline__ void eval(const Ctx& c, int il, double rr, double* o)
     {
         const Seg& g = c.sg[il];
         const double u = rr - g.r0;
         const double rrho = seg(g, u, P_RHO), rccon = seg(g, u, P_CCON), rxa2 = seg(g, u, P_XA2);
-        const double gg = seg(g, u, P_GRAV);
         const cd qaa = 1.0 + rxa2 * c.lno;
         const double dc = rccon * norm2(qaa);
         const double inv = 1.0 / (rr * rrho * dc);
         const double ri = (rrho * dc) * inv;
+        double gg = 0.0;
+        cd s = -(c.omega2 * rrho);
+        if (KIND != 0) {
+            gg = seg(g, u, P_GRAV);
+            s = s - 4.0 * (rrho * gg * ri);
+        }
         put(o, 0, conj(qaa) * ((rr * rrho) * inv));
         put(o, 1, c.omegai2 * (ri * ri));
-        put(o, 2, -(c.omega2 * rrho) - 4.0 * (rrho * gg * ri));
+        put(o, 2, s);
         put(o, 3, mk(ri, rrho));
         put(o, 4, mk(gg, (rr * dc) * inv));
     }
@@ -168,7 +177,7 @@ __device__ __forceinline__ FluidCoef fluid_amat(const LaneCtx& c, double)
     a.t21 = a.t22 = a.k22 = 0.0;
     if (KIND == 0) {
         a.t11 = mk(-rr.x);
-        a.s11 = got(c.p, 2) + 4.0 * (rr.y * gr.x * rr.x);
+        a.s11 = got(c.p, 2);
         return a;
     }
     const cd gz = gr.x * z;
