@@ -23,6 +23,7 @@
 #include <cooperative_groups.h>
 
 #include "ysg_kernels.h"
+#include "ysg_tables.cuh"
 
 namespace ysg {
 
@@ -53,7 +54,11 @@ __device__ __forceinline__ cd row_value(unsigned i, const TraceDev& td, const cd
 // 2^s - 1, entry m: exp(i m pi / 2^s); they do not depend on n), or those of
 // the last stage of n alone (tw[m] = exp(i m pi / (n/2)), for the two
 // passes); the taper per bin (module_fourier.f90:96-116); e^{eps t} per
-// sample.  Null pointers leave a table out.
+// sample.  Null pointers leave a table out.  Every entry is within 0.502 units
+// in the last place of the function of its (rounded) argument (ysg_tables.cuh).
+// With the library's sincos and exp, within 1.36 and 0.85 units, 400 receivers
+// of 16384 samples are 2.2e-16 off 64-bit arithmetic, with these 9.8e-17, for
+// 1.0 of 257 us.
 // ---------------------------------------------------------------------------
 __global__ void k_time_tables(int nstage, cd* __restrict__ tws, int nhalf, cd* __restrict__ tw, TaperDev f, int nbin,
                               double* __restrict__ filt, double ep, double dt, int nout, double* __restrict__ expt)
@@ -63,27 +68,32 @@ __global__ void k_time_tables(int nstage, cd* __restrict__ tws, int nhalf, cd* _
     if (tws && i < (1 << nstage) - 1) {
         const int s = 31 - __clz(i + 1), m = i + 1 - (1 << s);
         double sn, c;
-        sincos((double)m * (pi_d / (double)(1 << s)), &sn, &c);
+        table_sincos((double)m * (pi_d / (double)(1 << s)), &sn, &c);
         tws[i] = mk(c, sn);
     }
     if (tw && i < nhalf) {
         double sn, c;
-        sincos((double)i * (pi_d / (double)nhalf), &sn, &c);
+        table_sincos((double)i * (pi_d / (double)nhalf), &sn, &c);
         tw[i] = mk(c, sn);
     }
     if (filt && i < nbin) {
         double v = 1.0;
         if (!(f.w1 == 0.0 && f.w2 == 0.0 && f.w3 == 0.0 && f.w4 == 0.0)) {
-            const double w = (double)i * f.df;
+            const double w = __dmul_rn((double)i, f.df);
+            double x = -1.0, s, c;                          // angle on the flanks
             if (w < f.w1) v = 0.0;
-            else if (w < f.w2) v = 0.5 * (1.0 - cos(pi_d * (w - f.w1) / (f.w2 - f.w1)));
+            else if (w < f.w2) x = pi_d * (w - f.w1) / (f.w2 - f.w1);
             else if (w < f.w3) v = 1.0;
-            else if (w < f.w4) v = 0.5 * (1.0 - cos(pi_d * (f.w4 - w) / (f.w4 - f.w3)));
+            else if (w < f.w4) x = pi_d * (f.w4 - w) / (f.w4 - f.w3);
             else v = 0.0;
+            if (x >= 0.0) {
+                table_sincos(x, &s, &c);
+                v = 0.5 * (1.0 - c);
+            }
         }
         filt[i] = v;
     }
-    if (expt && i < nout) expt[i] = exp(ep * ((double)i * dt));
+    if (expt && i < nout) expt[i] = table_exp(ep * ((double)i * dt));
 }
 
 cudaError_t launch_time_tables(int nstage, cd* tws, int nhalf, cd* tw, const TaperDev& f, int nbin, double* filt,
