@@ -228,7 +228,7 @@ class KnotModel:
         in the library 0.1 ms."""
         import torch
 
-        if _plain(Y):
+        if _plain(Y) and Y.dim() == 2 and Y.shape[0] == self.nknot:
             y = Y.detach().contiguous()
             out = torch.empty_like(y)
             cols = y.shape[1] * (2 if y.is_complex() else 1)
