@@ -130,17 +130,22 @@ class _LayerSpline:
 def _plain(t) -> bool:
     """Whether t is an ordinary double or complex double tensor on the CPU whose
     operations nothing records or transforms (autograd, forward mode, vmap
-    and other functional transforms, tracing, dispatch modes)."""
+    and other functional transforms, tracing, dispatch modes).  Some of these are
+    only told by torch's private interface: where a version does not have it,
+    nothing is taken for plain."""
     import torch
 
     C = torch._C
-    return (type(t) is torch.Tensor and t.layout == torch.strided and t.device.type == "cpu"
-            and t.dtype in (torch.float64, torch.complex128) and not t.is_conj() and not t.is_neg()
-            and not (torch.is_grad_enabled() and t.requires_grad)
-            and not C._functorch.is_functorch_wrapped_tensor(t)
-            and torch.autograd.forward_ad.unpack_dual(t).tangent is None
-            and not torch.jit.is_tracing() and not torch.compiler.is_compiling()
-            and C._len_torch_dispatch_stack() == 0 and C._len_torch_function_stack() == 0)
+    try:
+        return (type(t) is torch.Tensor and t.layout == torch.strided and t.device.type == "cpu"
+                and t.dtype in (torch.float64, torch.complex128) and not t.is_conj() and not t.is_neg()
+                and not (torch.is_grad_enabled() and t.requires_grad)
+                and not C._functorch.is_functorch_wrapped_tensor(t)
+                and torch.autograd.forward_ad.unpack_dual(t).tangent is None
+                and not torch.jit.is_tracing() and not torch.compiler.is_compiling()
+                and C._len_torch_dispatch_stack() == 0 and C._len_torch_function_stack() == 0)
+    except AttributeError:
+        return False
 
 
 def _spline_fn():
