@@ -265,6 +265,13 @@ int ysg_set_schedule(ysg_handle *h, int sched);
  * each schedule from the last autotuning run (tune_ms may be NULL). */
 int ysg_last_schedule(ysg_handle *h, int *sched, float tune_ms[3]);
 
+/* Kernel form of the last solve stage by groups of degrees, per kind of solve:
+ * [0..2] spheroidal without gravity, Cowling, self-gravitating, [3] toroidal,
+ * [4] l = 0.  0 = the wide form (128 degrees per item, for lists that fill the
+ * GPU), 1 = the narrow one (32), -1 = no items of that kind, or a solve that
+ * did not run by groups. */
+int ysg_last_forms(ysg_handle *h, int form[5]);
+
 /* Device times in ms of the last event's stages, measured with CUDA events:
  * [0] Legendre table, [1] solves, [2] l-sum, [3] filter + inverse FFT +
  * post-processing.  For a single event (not a batch) the Legendre table is

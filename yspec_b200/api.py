@@ -25,6 +25,7 @@ from . import native as N
 # lengths of the arrays the engine fills (include/yspec_gpu.h)
 N_STAGE_TIMES = 4   # ysg_last_timings: legendre, solve, l-sum, time series
 N_SCHEDULES = 3     # ysg_last_schedule: tuning time of each batched-solver schedule
+N_GROUPS = 5        # ysg_last_forms: kinds of solves by groups of degrees
 
 
 def norms() -> dict:
@@ -161,6 +162,13 @@ class Engine:
         ms = (C.c_float * N_SCHEDULES)()
         N.check(N.lib().ysg_last_schedule(self.h, C.byref(s), ms), "last_schedule")
         return s.value, list(ms)
+
+    def last_forms(self) -> list[int]:
+        """Kernel form of the last solve by groups of degrees (0 wide, 1 narrow, -1 none): spheroidal
+        without gravity, Cowling and self-gravitating, toroidal, l = 0."""
+        f = (C.c_int * N_GROUPS)()
+        N.check(N.lib().ysg_last_forms(self.h, f), "last_forms")
+        return list(f)
 
     def upload(self, model: Model) -> None:
         """Upload a model: a Model read from a deck, or any object whose view()

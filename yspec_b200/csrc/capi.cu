@@ -1218,6 +1218,16 @@ int ysg_last_schedule(ysg_handle* h, int* sched, float* tune_ms)
     return YSG_OK;
 }
 
+static_assert(NGROUP == 5, "ysg_last_forms' form[] holds 5 entries (yspec_gpu.h)");
+
+int ysg_last_forms(ysg_handle* h, int* form)
+{
+    if (!h || !form) return YSG_ERR_ARG;
+    const bool by_groups = h->solver == 1 && h->groups && h->cur_sched == 2;
+    for (int k = 0; k < NGROUP; k++) form[k] = by_groups && h->gitems[k] > 0 ? h->gform[k] : -1;
+    return YSG_OK;
+}
+
 int ysg_get_stream(ysg_handle* h, void** stream)
 {
     if (!h || !stream) return YSG_ERR_ARG;
