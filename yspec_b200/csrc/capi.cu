@@ -1448,7 +1448,8 @@ int ysg_event_gradient(ysg_handle* h, const ysg_event* ev, const ysg_time* tm, c
     const int gkind[2] = {GROUP_SPH0 + ev->grav, GROUP_TOR};
     long long gitems[2] = {};
     int gblk[2] = {};
-    const size_t glane = ((size_t)nmax + ncmax) * (14 * sizeof(cd) + sizeof(double));
+    // logs of a lane: a state of the kind's own components and a factor per step
+    auto glane = [&](int kind) { return ((size_t)nmax + ncmax) * (group_adj_states(kind) * sizeof(cd) + sizeof(double)); };
     const size_t grad_b = (size_t)nw * gmax * (4 * sizeof(cd) + sizeof(double) + sizeof(int)) +
                           (size_t)nw * 32 * adj_step_bytes(RAD_PIECE_STEPS) + 4096;
     size_t log_bytes = 0, T = 0, Tr = 0;
@@ -1466,7 +1467,7 @@ int ysg_event_gradient(ysg_handle* h, const ysg_event* ev, const ysg_time* tm, c
         }
         auto total = [&]() {
             size_t b = need;
-            for (int q = 0; q < 2; q++) b += (size_t)gblk[q] * group_adj_threads(gkind[q]) * glane;
+            for (int q = 0; q < 2; q++) b += (size_t)gblk[q] * group_adj_threads(gkind[q]) * glane(gkind[q]);
             return b;
         };
         while (over(total()) && (gblk[0] > 1 || gblk[1] > 1))
@@ -1540,10 +1541,10 @@ int ysg_event_gradient(ysg_handle* h, const ysg_event* ev, const ysg_time* tm, c
         return w;
     };
     // the states and rescaling factors alone, for the sweeps by groups
-    auto states_of = [&](size_t nt, int n) {
+    auto states_of = [&](size_t nt, int n, int states) {
         AdjStepArrays a{};
         a.n = n;
-        a.y = reinterpret_cast<cd*>(take((size_t)n * 14 * nt * sizeof(cd)));
+        a.y = reinterpret_cast<cd*>(take((size_t)n * states * nt * sizeof(cd)));
         a.f = reinterpret_cast<double*>(take((size_t)n * nt * sizeof(double)));
         return a;
     };
@@ -1599,8 +1600,8 @@ int ysg_event_gradient(ysg_handle* h, const ysg_event* ev, const ysg_time* tm, c
             const size_t nt = (size_t)gblk[q] * group_adj_threads(gkind[q]);
             AdjLogs wg{};
             wg.nthreads = (int)nt;
-            wg.s = states_of(nt, nmax);
-            wg.c = states_of(nt, ncmax);
+            wg.s = states_of(nt, nmax, group_adj_states(gkind[q]));
+            wg.c = states_of(nt, ncmax, group_adj_states(gkind[q]));
             int launched = 0;
             CK(launch_group_adj(gkind[q], h->kn.as<Knot>(), h->sg.as<Seg>(), h->hdr_dev.as<ModelHdr>(),
                                 h->evdev.as<EventDev>(), u, h->acoefb.as<cd>(), h->agoff.as<long long>() + 2 * q,

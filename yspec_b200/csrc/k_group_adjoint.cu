@@ -247,6 +247,7 @@ struct AdjMem {
     static constexpr int NW = 1, NL = NL_, SLOTS = SLOTS_, NT = 32 * NL_;
     static constexpr int SB = NT / 6 < 8 ? NT / 6 : 8;
     static constexpr bool KEEP_R = true;
+    static constexpr int LOG_N = NMAX;
     static constexpr int ROWS = NMAX, OWN = NMAX;
     double pt[SB * 6][PT];
     cd ex[1][1][32];
@@ -373,7 +374,7 @@ __device__ __noinline__ void group_rev(Group& g, const GroupLog& lg, int at, int
 #pragma unroll
                 for (int k = 0; k < N; k++) {
                     cd v = mk(0.0);
-                    if (live) v = lg.y[((size_t)q * GLOG_N + k) * lg.stride];
+                    if (live) v = lg.y[((size_t)q * Mem::LOG_N + k) * lg.stride];
                     yt[k] = v;
                     Y[0][k] = v;
                 }
@@ -970,7 +971,7 @@ __global__ void __launch_bounds__(32 * NL, MINB) k_gadj_tor(AdjArgs a)
 // radius, size, interval and rescaling factor in the same arrays.
 struct RadLog {
     cd* y;                        // gmax x 4
-    double* r;                    // gmax x 2
+    double* r;                    // gmax
     int* i;                       // gmax
     int gmax;
 };
@@ -1288,14 +1289,20 @@ struct AdjKernel {
     int threads;
     size_t smem;
     int width;
+    int states;                   // components of a logged state
 };
+template <class Mem>
+AdjKernel adj_kernel_of(AdjFn f)
+{
+    return {f, Mem::NT, sizeof(Mem), 32 * Mem::NL, Mem::LOG_N};
+}
 AdjKernel adj_kernel(int kind)
 {
     switch (kind) {
-        case GROUP_SPH2: return {k_gadj_sph<2, GADJ_NL, 8 / GADJ_NL>, 32 * GADJ_NL, sizeof(SphAdjMem<2, GADJ_NL>), 32 * GADJ_NL};
-        case GROUP_SPH1: return {k_gadj_sph<1, GADJ_NL, 8 / GADJ_NL>, 32 * GADJ_NL, sizeof(SphAdjMem<1, GADJ_NL>), 32 * GADJ_NL};
-        case GROUP_SPH0: return {k_gadj_sph<0, GADJ_NL, 8 / GADJ_NL>, 32 * GADJ_NL, sizeof(SphAdjMem<0, GADJ_NL>), 32 * GADJ_NL};
-        default: return {k_gadj_tor<GADJ_NL, 16 / GADJ_NL>, 32 * GADJ_NL, sizeof(TorAdjMem<GADJ_NL>), 32 * GADJ_NL};
+        case GROUP_SPH2: return adj_kernel_of<SphAdjMem<2, GADJ_NL>>(k_gadj_sph<2, GADJ_NL, 8 / GADJ_NL>);
+        case GROUP_SPH1: return adj_kernel_of<SphAdjMem<1, GADJ_NL>>(k_gadj_sph<1, GADJ_NL, 8 / GADJ_NL>);
+        case GROUP_SPH0: return adj_kernel_of<SphAdjMem<0, GADJ_NL>>(k_gadj_sph<0, GADJ_NL, 8 / GADJ_NL>);
+        default: return adj_kernel_of<TorAdjMem<GADJ_NL>>(k_gadj_tor<GADJ_NL, 16 / GADJ_NL>);
     }
 }
 
@@ -1305,6 +1312,8 @@ AdjKernel adj_kernel(int kind)
 int group_adj_width(int kind) { return adj_kernel(kind).width; }
 
 int group_adj_threads(int kind) { return adj_kernel(kind).threads; }
+
+int group_adj_states(int kind) { return adj_kernel(kind).states; }
 
 int group_adj_blocks(int kind)
 {

@@ -215,6 +215,7 @@ struct GroupMem {
     static constexpr int NT = 32 * NW * NL;        // threads
     static constexpr int SB = NT / 6;              // steps per batch of points
     static constexpr bool KEEP_R = false;          // the points' radii are not kept
+    static constexpr int LOG_N = NMAX;             // components of a logged state
     static constexpr int ROWS = NMAX + (NW > 1 ? 1 : 0);   // the last row takes the empty own slots
     static constexpr int OWN = (NMAX + NW - 1) / NW;
     double pt[SB * 6][PT];                         // points of the batch
@@ -502,9 +503,9 @@ struct StageVec {
 };
 
 // Log of the states before every step of a walk (and the rescaling factor
-// after it), entry (step, component) of the lanes of a launch side by side;
-// the pointers are the thread's own.
-constexpr int GLOG_N = 14;
+// after it), entry (step, component) of the lanes of a launch side by side,
+// LOG_N components of the largest system of the kernel; the pointers are the
+// thread's own.
 struct GroupLog {
     cd* y;
     double* f;
@@ -573,7 +574,7 @@ __device__ __noinline__ void group_walk(Group& g, int i1, int i2, double r1, dou
                 // streaming stores: only the reverse pass reads them back
 #pragma unroll
                 for (int k = 0; k < NO; k++)
-                    __stcs(reinterpret_cast<double2*>(lg->y + ((size_t)lq * GLOG_N + k) * lg->stride),
+                    __stcs(reinterpret_cast<double2*>(lg->y + ((size_t)lq * Mem::LOG_N + k) * lg->stride),
                            make_double2(y[k].x, y[k].y));
             }
             const double(*p)[PT] = M.pt + s * 6;

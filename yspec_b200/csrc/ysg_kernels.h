@@ -189,6 +189,7 @@ cudaError_t launch_solve_adjoint(const Knot* kn, const Seg* sg, const ModelHdr* 
 // minors and the toroidal solutions); grad and status as launch_solve_adjoint.
 int group_adj_width(int kind);
 int group_adj_threads(int kind);
+int group_adj_states(int kind);                   // components of a logged state
 int group_adj_blocks(int kind);                   // resident grid, 0 on failure
 cudaError_t launch_group_adj(int kind, const Knot* kn, const Seg* sg, const ModelHdr* mh, const EventDev* ev,
                              const UnitDirs& u, const cd* coefb, const long long* off, long long nitems,
