@@ -250,7 +250,6 @@ struct AdjMem {
     static constexpr int LOG_N = NMAX;
     static constexpr int ROWS = NMAX, OWN = NMAX;
     double pt[SB * 6][PT];
-    cd ex[1][1][32];
     cd slot[SLOTS > 0 ? SLOTS : 1][SLOTS > 0 ? NMAX : 1][SLOTS > 0 ? NT : 1];
     double pb[NL][SB * 6][ADJ_NV];
     double vb[SB * 6][NPARAM];
@@ -260,7 +259,6 @@ struct AdjMem {
     int sil[SB];
     int i1[32];
     double rt[32];
-    unsigned flag[4][2];
     unsigned long long item;
 };
 

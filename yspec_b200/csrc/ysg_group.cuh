@@ -225,7 +225,7 @@ struct GroupMem {
     int sil[SB];                                   // intervals
     int i1[32];
     double rt[32];
-    unsigned flag[4][2];                           // per warp: lanes with every / any own component out of range
+    unsigned flag[NW][2];                          // per warp: lanes with every / any own component out of range
     unsigned long long item;
 };
 
@@ -304,10 +304,7 @@ __device__ __forceinline__ Own<Split<Sys, NW>::NO> own_rows(int warp)
         for (int k = 0; k < NO; k++) o.row[k] = k;
         return o;
     }
-    unsigned m = Split<Sys, NW>::mask(0);
-#pragma unroll
-    for (int w = 1; w < NW; w++)
-        if (warp == w) m = Split<Sys, NW>::mask(w);
+    unsigned m = warp == 0 ? Split<Sys, NW>::mask(0) : Split<Sys, NW>::mask(1);
 #pragma unroll
     for (int k = 0; k < NO; k++) {
         o.row[k] = m ? __ffs(m) - 1 : Mem::ROWS - 1;
@@ -357,15 +354,9 @@ __device__ __forceinline__ void rhs_part(const LaneCtx& lc, const cd (*ex)[32], 
 template <class Sys, int NW>
 __device__ __forceinline__ void rhs_own(int warp, const LaneCtx& lc, const cd (*ex)[32], int lane, const cd* yt, cd* d)
 {
-    if (NW == 1 || warp == 0) {
-        rhs_part<Sys, NW, 0>(lc, ex, lane, yt, d);
-    } else if (NW == 2 || warp == 1) {
-        rhs_part<Sys, NW, 1 % NW>(lc, ex, lane, yt, d);
-    } else if (warp == 2) {
-        rhs_part<Sys, NW, 2 % NW>(lc, ex, lane, yt, d);
-    } else {
-        rhs_part<Sys, NW, 3 % NW>(lc, ex, lane, yt, d);
-    }
+    static_assert(NW <= 2, "a part of the right-hand side per warp");
+    if (NW == 1 || warp == 0) rhs_part<Sys, NW, 0>(lc, ex, lane, yt, d);
+    else rhs_part<Sys, NW, NW - 1>(lc, ex, lane, yt, d);
 }
 
 __device__ __forceinline__ int hi_abs(double x) { return __double2hiint(x) & 0x7fffffff; }
@@ -485,6 +476,14 @@ __device__ __noinline__ int walk_fill(const Group& g, Walk& w)
     return nb;
 }
 
+// The exchange's buffer b; none where a warp holds all components.
+template <class Mem>
+__device__ __forceinline__ const cd (*exchange(const Mem& M, int b))[32]
+{
+    if constexpr (Mem::NW > 1) return M.ex[b];
+    else return nullptr;
+}
+
 // A stage vector of the own components: in registers, or (SM) in the
 // thread's column of a shared-memory slot.
 template <class Mem, int NO, bool SM, int WHICH>
@@ -563,7 +562,7 @@ __device__ __noinline__ void group_walk(Group& g, int i1, int i2, double r1, dou
                     if (LOG) g.jq = lq;
                 }
                 nact = __popc(__ballot_sync(FULL, started));
-                if (NW > 1) {
+                if constexpr (NW > 1) {
                     publish(M.ex[0], own, lane, y);
                     gsync<Mem>();
                 }
@@ -596,7 +595,7 @@ __device__ __noinline__ void group_walk(Group& g, int i1, int i2, double r1, dou
                     const double h = *(volatile double*)&M.sh[s];
                     cd d[NO];
                     lc.p = p[st];
-                    rhs_own<Sys, NW>(warp, lc, M.ex[NW > 1 ? st & 1 : 0], lane, yt, d);
+                    rhs_own<Sys, NW>(warp, lc, exchange(M, st & 1), lane, yt, d);
                     if (st == 0) {
 #pragma unroll
                         for (int k = 0; k < NO; k++) {
@@ -633,9 +632,11 @@ __device__ __noinline__ void group_walk(Group& g, int i1, int i2, double r1, dou
 #pragma unroll
                         for (int k = 0; k < NO; k++) y[k] = cmac(y[k], (512.0 / 1771.0) * h, d[k]);
                     }
-                    if (NW > 1 && st < 5) {
-                        publish(M.ex[(st + 1) & 1], own, lane, yt);
-                        gsync<Mem>();
+                    if constexpr (NW > 1) {
+                        if (st < 5) {
+                            publish(M.ex[(st + 1) & 1], own, lane, yt);
+                            gsync<Mem>();
+                        }
                     }
                 }
             } else {
@@ -650,14 +651,14 @@ __device__ __noinline__ void group_walk(Group& g, int i1, int i2, double r1, dou
                 }
 #pragma unroll 1
                 for (int st = 5; st >= 0; st--) {
-                    if (NW > 1) {
+                    if constexpr (NW > 1) {
                         publish(M.ex[st & 1], own, lane, yt);
                         gsync<Mem>();
                     }
                     const double h = *(volatile double*)&M.sh[s];
                     cd d[NO];
                     lc.p = p[st];
-                    rhs_own<Sys, NW>(warp, lc, M.ex[NW > 1 ? st & 1 : 0], lane, yt, d);
+                    rhs_own<Sys, NW>(warp, lc, exchange(M, st & 1), lane, yt, d);
                     if (st == 5) {
 #pragma unroll
                         for (int k = 0; k < NO; k++) {
@@ -711,10 +712,10 @@ __device__ __noinline__ void group_walk(Group& g, int i1, int i2, double r1, dou
             for (int k = 0; k < NO; k++) mx = max(mx, max(hi_abs(y[k].x), hi_abs(y[k].y)));
             double factor = 1.0;
             const bool small = started && mx < 0x3BC79CA1, big = started && mx > 0x4415AF1D;
-            if (NW > 1 && !TR) publish(M.ex[0], own, lane, y);
+            if constexpr (NW > 1 && !TR) publish(M.ex[0], own, lane, y);
             if (gany<Mem>(small || big)) {
                 unsigned sb = __ballot_sync(FULL, small), bb = __ballot_sync(FULL, big);
-                if (NW > 1) {
+                if constexpr (NW > 1) {
                     if (lane == 0) {
                         M.flag[g.warp][0] = sb;
                         M.flag[g.warp][1] = bb;
@@ -735,7 +736,7 @@ __device__ __noinline__ void group_walk(Group& g, int i1, int i2, double r1, dou
                     scale += s1 ? 1 : -1;
 #pragma unroll
                     for (int k = 0; k < NO; k++) y[k] = y[k] * f;
-                    if (NW > 1 && !TR) publish(M.ex[0], own, lane, y);
+                    if constexpr (NW > 1 && !TR) publish(M.ex[0], own, lane, y);
                 }
                 gsync<Mem>();
             }
@@ -748,7 +749,7 @@ __device__ __noinline__ void group_walk(Group& g, int i1, int i2, double r1, dou
         // overflow.
         if (NW == 1) bsync<Mem>();
     }
-    if (NW > 1 && TR) {              // the other form publishes after every step
+    if constexpr (NW > 1 && TR) {    // the other form publishes after every step
         publish(M.ex[0], own, lane, y);
         gsync<Mem>();
     }
@@ -773,7 +774,7 @@ __device__ __forceinline__ void group_join_rest(Group& g, int last, cd* y, const
         for (int k = 0; k < Split<Sys, NW>::NO; k++) y[k] = start[k];
         g.started = true;
     }
-    if (NW > 1) {
+    if constexpr (NW > 1) {
         publish(group_mem<Mem>().ex[0], own_rows<Sys, NW, Mem>(g.warp), g.lane, y);
         gsync<Mem>();
     }
