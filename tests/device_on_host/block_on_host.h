@@ -1,7 +1,7 @@
 // block_on_host.h -- run one thread block of device code on the CPU.
 //
-// Every thread of the block is a coroutine (ucontext); the warp and block
-// collectives suspend it until all threads they join have arrived.  Device
+// Every thread of the block is a coroutine with a stack of its own; the warp and
+// block collectives suspend it until all threads they join have arrived.  Device
 // qualifiers become nothing, the explicitly rounded intrinsics the plain
 // operations.  A thread that leaves a collective out hangs no GPU here: the
 // scheduler sees that nobody advances and aborts.
@@ -12,7 +12,6 @@
 #include <cstdlib>
 #include <cstring>
 #include <functional>
-#include <ucontext.h>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -38,8 +37,34 @@ namespace block {
 constexpr int MAX_THREADS = 128;
 constexpr size_t STACK = 1 << 20;
 
+#if !defined(__x86_64__)
+#error "the switch between stacks is written for x86-64"
+#endif
+// Saves the callee-saved registers and the stack pointer, and takes up another stack.
+extern "C" void block_switch_stack(void** save, void* to);
+asm(R"(
+    .text
+    .globl block_switch_stack
+block_switch_stack:
+    pushq %rbp
+    pushq %rbx
+    pushq %r12
+    pushq %r13
+    pushq %r14
+    pushq %r15
+    movq %rsp, (%rdi)
+    movq %rsi, %rsp
+    popq %r15
+    popq %r14
+    popq %r13
+    popq %r12
+    popq %rbx
+    popq %rbp
+    ret
+)");
+
 struct Fiber {
-    ucontext_t c;
+    void* sp;
     std::vector<char> stack;
     bool done;
 };
@@ -47,7 +72,7 @@ struct Barrier {
     int gen = 0, n = 0;
 };
 inline Fiber fiber[MAX_THREADS];
-inline ucontext_t scheduler;
+inline void* scheduler;
 inline int nthreads, cur;
 inline unsigned block_id, grid_size;
 inline Barrier warp_bar[MAX_THREADS / 32], block_bar;
@@ -58,7 +83,7 @@ inline std::function<void()> body;
 inline void yield()
 {
     const int me = cur;
-    swapcontext(&fiber[me].c, &scheduler);
+    block_switch_stack(&fiber[me].sp, scheduler);
     cur = me;
 }
 inline void wait(Barrier& b, int need)
@@ -89,11 +114,11 @@ inline void run(int threads, unsigned id, unsigned grid, std::function<void()> f
     body = f;
     for (int t = 0; t < threads; t++) {
         fiber[t].stack.resize(STACK);
-        getcontext(&fiber[t].c);
-        fiber[t].c.uc_stack.ss_sp = fiber[t].stack.data();
-        fiber[t].c.uc_stack.ss_size = STACK;
-        fiber[t].c.uc_link = nullptr;
-        makecontext(&fiber[t].c, entry, 0);
+        // as block_switch_stack leaves it: six registers, the return address, an aligned frame
+        void** top = reinterpret_cast<void**>(((size_t)fiber[t].stack.data() + STACK) & ~(size_t)63) - 1;
+        *--top = reinterpret_cast<void*>(&entry);
+        for (int r = 0; r < 6; r++) *--top = nullptr;
+        fiber[t].sp = top;
         fiber[t].done = false;
     }
     for (int left = threads; left;) {
@@ -102,7 +127,7 @@ inline void run(int threads, unsigned id, unsigned grid, std::function<void()> f
         for (int t = 0; t < threads; t++) {
             if (fiber[t].done) continue;
             cur = t;
-            swapcontext(&scheduler, &fiber[t].c);
+            block_switch_stack(&scheduler, fiber[t].sp);
             left += !fiber[t].done;
         }
         if (left && progress == before) {
