@@ -281,10 +281,16 @@ int ysg_last_forms(ysg_handle *h, int form[5]);
 int ysg_last_timings(ysg_handle *h, float ms[4]);
 
 /* Counters of the last solve stage: number of (omega,l) pairs and the
- * algorithmic FP64 flop count of the stepping work actually performed (solves
- * that events of a batch share, those that differ in the moment tensor
- * alone, count once). */
+ * algorithmic FP64 flop count of the steps taken, a coefficient matrix for every
+ * pair, step and stage (solves that events of a batch share, those that differ
+ * in the moment tensor alone, count once). */
 int ysg_last_work(ysg_handle *h, double *pairs, double *flops);
+
+/* FP64 flops of the same steps as the kernels execute them: by groups of
+ * degrees the l-independent part of a coefficient matrix is formed once per
+ * item, where ysg_last_work counts it for every pair.  Equal to its count for
+ * the other forms. */
+int ysg_last_executed(ysg_handle *h, double *flops);
 
 /* Kernels of this library enqueued since the last ysg_event_prepare (or
  * ysg_event_run / ysg_batch_run), autotuning runs excluded. */

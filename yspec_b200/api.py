@@ -317,6 +317,12 @@ class Engine:
         N.check(N.lib().ysg_last_work(self.h, C.byref(p), C.byref(f)), "work")
         return p.value, f.value
 
+    def executed_flops(self) -> float:
+        """FP64 flops of the last solve stage's steps as the kernels execute them."""
+        f = C.c_double()
+        N.check(N.lib().ysg_last_executed(self.h, C.byref(f)), "executed_flops")
+        return f.value
+
 
 def fp64_peak_tflops(device: int = 0) -> float:
     """Measured FP64 FMA throughput of the device (TFLOP/s)."""

@@ -64,6 +64,27 @@ const double kStepFlops[NSYS_COUNT] = {
     6 * 666.0 + 88.0 * 14,   // b-vector, self-gravitation
 };
 
+// The same for the solves by groups of degrees, as the kernels execute them:
+// per lane the right-hand side without the l-independent part of the
+// coefficient matrix, and that part (a point of ysg_group.cuh) once per item
+// instead of once per lane.  Hand tallies of the same expressions (of the
+// 666 flops of a self-gravitating solid 163 are the matrix: 151 for the point,
+// 13 per lane).  The l = 0 solves form no points (ysg_radial.cuh).
+struct GroupFlops {
+    double lane, point;
+};
+const GroupFlops kGroupRhsFlops[NSYS_COUNT] = {
+    {45.0, 43.0},            // toroidal
+    {177.0, 0.0},            // radial
+    {43.0, 57.0},            // fluid minors, no gravity / Cowling
+    {145.0, 145.0},          // b-vector, no gravity / Cowling
+    {155.0, 145.0},          // solid minors, no gravity / Cowling
+    {173.0, 67.0},           // fluid minors, self-gravitation
+    {516.0, 151.0},          // solid minors, self-gravitation
+    {516.0, 151.0},          // b-vector, self-gravitation
+};
+const double kStepComponents[NSYS_COUNT] = {2, 2, 2, 4, 5, 5, 14, 14};
+
 // Work of a pair outside the stepping (start level, start vectors, minor
 // algebra, source vectors), for the scheduler's cost model only.
 constexpr double kPairBaseFlops = 2.0e4;
@@ -162,7 +183,7 @@ struct ysg_handle {
     bool capturing = false;          // enqueue_* run under stream capture
     float ms[4] = {0, 0, 0, 0};
     double h2d = 0.0, d2h = 0.0;     // bytes moved since the last prepare
-    double pairs = 0.0, flops = 0.0;
+    double pairs = 0.0, flops = 0.0, executed = 0.0;
 };
 
 // CUDA failures return YSG_ERR_CUDA and leave the runtime's error name and
@@ -877,6 +898,29 @@ int enqueue_chains(ysg_handle* h, int nev, int ns)
     return YSG_OK;
 }
 
+// Flops of the last solve stage's steps as executed, from the step counters.
+// A point's share is that of an item whose lanes are all filled.
+double executed_flops(const ysg_handle* h, const unsigned long long* steps)
+{
+    const bool by_groups = h->solver == 1 && h->groups && h->cur_sched == 2;
+    double fl = 0.0;
+    for (int q = 0; q < NSYS_COUNT; q++) {
+        if (!by_groups) {
+            fl += (double)steps[q] * kStepFlops[q];
+            continue;
+        }
+        // the narrowest form among the kinds that step this class (2 - 4: with and without Cowling's gravity)
+        int width = 1;
+        for (int k : {q == 0 ? GROUP_TOR : q == 1 ? GROUP_RAD : q >= 5 ? GROUP_SPH2 : GROUP_SPH1, q >= 2 && q <= 4 ? GROUP_SPH0 : NGROUP})
+            if (k != NGROUP && h->gitems[k] > 0) {
+                const int wk = group_form_width(k, h->gform[k]);
+                width = width == 1 ? wk : std::min(width, wk);
+            }
+        fl += (double)steps[q] * (6.0 * (kGroupRhsFlops[q].lane + kGroupRhsFlops[q].point / width) + 88.0 * kStepComponents[q]);
+    }
+    return fl;
+}
+
 // Wait for the stream, read the solve counters and the status word.
 int finish(ysg_handle* h, int nev, bool spectra, bool traces)
 {
@@ -891,6 +935,7 @@ int finish(ysg_handle* h, int nev, bool spectra, bool traces)
         double fl = 0.0;
         for (int q = 0; q < NSYS_COUNT; q++) fl += (double)w[q] * kStepFlops[q];
         h->flops = fl;
+        h->executed = executed_flops(h, w);
         double pairs = 0.0;
         for (int e = 0; e < nev; e++) {
             const EventDev& d = h->slots[(size_t)e].pev;
@@ -1651,7 +1696,7 @@ int ysg_event_gradient(ysg_handle* h, const ysg_event* ev, const ysg_time* tm, c
     CK(cudaEventElapsedTime(&t[1], h->ev[3], h->ev[4]));
     for (int i = 0; i < 4; i++) h->ms[i] = t[i];
     h->pairs = (double)L * nw;
-    h->flops = 0.0;
+    h->flops = h->executed = 0.0;
     if (status) return YSG_ERR_LIMIT;
     // dL/dc[i][p][k] -> knot values and spline second derivatives, through
     // the segment formulas of build_tables
@@ -1878,6 +1923,13 @@ int ysg_last_work(ysg_handle* h, double* pairs, double* flops)
     if (!h) return YSG_ERR_ARG;
     if (pairs) *pairs = h->pairs;
     if (flops) *flops = h->flops;
+    return YSG_OK;
+}
+
+int ysg_last_executed(ysg_handle* h, double* flops)
+{
+    if (!h || !flops) return YSG_ERR_ARG;
+    *flops = h->executed;
     return YSG_OK;
 }
 
