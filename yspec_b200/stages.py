@@ -91,7 +91,7 @@ def main(argv=None) -> None:
                 eng.run(evs[0])
             wall = time.perf_counter() - t
             ms = eng.timings()
-            pairs, fl = eng.work()
+            pairs, fl = eng.work()[0], eng.executed_flops()
             sched = eng.last_schedule()[0] if a.solver == "batched" else "-"
             print(f"{a.config} {a.solver} sched {sched} rep{rep}: wall {wall:.3f} s  stages (ms) "
                   f"legendre {ms[0]:.3f} solve {ms[1]:.3f} lsum {ms[2]:.3f} ifft {ms[3]:.3f}  "
