@@ -275,7 +275,7 @@ def gradient_check(local: int) -> dict:
             "forward_s": min(fwd), "gradient_s": min(bwd), "gradient_over_forward": min(bwd) / min(fwd),
             "reverse_sweeps_ms": min(sweeps), "backend": syn.last_method,
             "method": "reverse mode: trace adjoint through the time-stage and l-sum transposes, discrete "
-                      "adjoint of every (omega, l) solve (k_solve_adjoint), autograd through the model chain",
+                      "adjoint of every (omega, l) solve (k_gadj_sph, k_gadj_tor, k_gadj_rad), autograd through the model chain",
             "fd_rel_err": max(errs), "fd_check": "central differences along 20 random directions, step 1e-3"}
 
 

@@ -23,12 +23,12 @@
 // contraction with the coefficients and the transposed product, about four
 // forward solves in all, at 8 warps per SM.  Of the cycles between two
 // instructions of a warp (31,003 pairs) 2.8 wait for the block's other warps
-// (the degrees that start deeper walk on alone), 2.2 for the logged states
+// (the degrees that start deeper walk on alone), 2.0 for the logged states
 // and the stage inputs (6 x 14 components per lane: local memory, held by
 // the L2), 1.8 for the FP64 pipe's latency and 0.8 for instructions.
-// Measured: 31,003 pairs 173 ms with a thread per pair, 13.4 ms here; their
+// Measured: 31,003 pairs 173 ms with a thread per pair, 11.9 ms here; their
 // l = 0 sweep 64 ms with a thread per frequency, 1.06 ms here; the gradient
-// call of a 200-knot ocean deck with 121 degrees 89 -> 5.9 ms.
+// call of a 200-knot ocean deck with 121 degrees 89 -> 5.7 ms.
 // Kernels:
 //   k_gadj_sph   spheroidal pairs, a degree per lane, NL warps per item
 //   k_gadj_tor   toroidal pairs

@@ -125,7 +125,7 @@ cudaError_t launch_time_tables(int nstage, cd* tws, int nhalf, cd* tw, const Tap
 // Positions are stored at p ^ ((p >> 3) & 7), so that 8 neighbouring threads
 // use different banks in every round, also in the first, where each has 8
 // consecutive values.  400 receivers, 1200 rows of 16384 and 7202 samples
-// kept: 254 us (the two passes in 16 MiB of rows, twiddles by sincos: 1286);
+// kept: 257 us (the two passes in 16 MiB of rows, twiddles by sincos: 1286);
 // half the issue slots are used, the rest wait for twiddles from the L2 and
 // at the rounds' barriers.  Tiles of 2048 take 5 us more (128 threads) or 100
 // (256), 512 threads on a tile 27.

@@ -20,7 +20,7 @@
 //       cost-sorted list (k_schedule.cu), persistent, a warp fetching 32
 //       consecutive entries at a time.  For models that cannot be solved by
 //       groups (a core boundary that is not a double knot); the others take
-//       k_group_adjoint.cu (31,003 pairs: 173 ms here, 13.4 ms there).
+//       k_group_adjoint.cu (31,003 pairs: 173 ms here, 11.9 ms there).
 //
 // Complex adjoints follow one convention throughout: for a real L and a
 // complex z, zb = dL/dRe z - i dL/dIm z, so dL = Re(sum zb dz) and a

@@ -518,10 +518,10 @@ struct GroupLog {
 // result.  With a start vector (`start`, own components), the lane's vector
 // is replaced by it when the walk reaches the lane's start level.
 //
-// The own stage vectors are held in registers: after
-// the third derivative the inputs of stages 5 and 6 and the result are
+// After the third derivative the inputs of stages 5 and 6 and the result are
 // carried as partial sums, so at most four vectors are live beside the
-// derivative.
+// derivative: y, the stage input and it in registers, the two partial sums
+// (v1, v2) in registers or, with SLOTS, in shared memory.
 template <class Sys, class Point, bool TR, class Mem, bool LOG = false>
 __device__ __noinline__ void group_walk(Group& g, int i1, int i2, double r1, double r2, cd* yio, const cd* start,
                                         const GroupLog* lg = nullptr, int at = 0)
@@ -577,11 +577,10 @@ __device__ __noinline__ void group_walk(Group& g, int i1, int i2, double r1, dou
                            make_double2(y[k].x, y[k].y));
             }
             const double(*p)[PT] = M.pt + s * 6;
-                            // One copy of the right-hand side in the code, the stage
-            // combinations by case: six copies would overflow the
-            // instruction cache, the stage vectors stay in registers.  The
-            // step size is read again every stage, so that its products with
-            // the weights are not all held in registers over the stages.
+            // One copy of the right-hand side in the code, the stage combinations
+            // by case: six copies would overflow the instruction cache.  The step
+            // size is read again every stage, so that its products with the
+            // weights are not all held in registers over the stages.
             StageVec<Mem, NO, TR ? (Mem::SLOTS > 0) : (Mem::SLOTS > 1), 0> v1;
             StageVec<Mem, NO, TR ? (Mem::SLOTS > 1) : (Mem::SLOTS > 0), 1> v2;
             cd yt[NO];

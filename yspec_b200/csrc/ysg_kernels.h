@@ -47,7 +47,7 @@ cudaError_t launch_solve_kernel(int kid, const Knot* kn, const Seg* sg, const Mo
                                 int item0, int item_end, int* counter, unsigned long long* work,
                                 int nblocks, cudaStream_t st);
 
-// K1 by groups of 32 degrees of one frequency (k_solve_group.cu), one list
+// K1 by groups of 128 or 32 degrees of one frequency (k_solve_group.cu), one list
 // of items per kind: the three gravity settings of the spheroidal solves
 // (GROUP_SPH0 + grav), the toroidal and the l = 0 ones.  For events with
 // the source and the receivers above the core.
@@ -60,8 +60,8 @@ long long group_items(int lmin, int lmax, int nw, int grav, int kind, int width)
 int group_blocks(int kind, int form);                                   // resident grid, 0 on failure
 // Bytes of the ordering work space of a list (used when nitems exceeds the resident grid).
 size_t group_order_bytes(long long nitems);
-// off: items of the events before e (nev + 1 entries); tt (nknot + 1
-// entries): sum of length / alpha over the intervals below knot k; counter
+// off: items of the events before e (nev + 1 entries); tt (nknot + 2
+// entries, 1-based): sum of length / alpha over the intervals below knot k; counter
 // is reset here.  *launched receives the kernels enqueued.
 cudaError_t launch_group(int kind, int form, const Knot* kn, const Seg* sg, const ModelHdr* mh, const EventDev* evs,
                          cd* const* coefs, const long long* off, int nev, long long nitems, const double* tt,
