@@ -57,26 +57,27 @@ __device__ __forceinline__ cd row_value(unsigned i, const TraceDev& td, const cd
 // sample.  Null pointers leave a table out.  Every entry is within 0.502 units
 // in the last place of the function of its (rounded) argument (ysg_tables.cuh).
 // With the library's sincos and exp, within 1.36 and 0.85 units, 400 receivers
-// of 16384 samples are 2.2e-16 off 64-bit arithmetic, with these 9.8e-17, for
-// 1.0 of 257 us.
+// of 16384 samples are 2.2e-16 off 64-bit arithmetic, with these 9.8e-17.  A row of
+// blocks per table: the functions are long dependent chains, one after the other
+// in a thread they took 2 us more (256.9 against 254.7 us for the whole call).
 // ---------------------------------------------------------------------------
 __global__ void k_time_tables(int nstage, cd* __restrict__ tws, int nhalf, cd* __restrict__ tw, TaperDev f, int nbin,
                               double* __restrict__ filt, double ep, double dt, int nout, double* __restrict__ expt)
 {
     const double pi_d = (double)3.14159265358979323846f;   // nrtype.f90 pi_d (single-precision literal)
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (tws && i < (1 << nstage) - 1) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, table = blockIdx.y;
+    if (table == 0 && tws && i < (1 << nstage) - 1) {
         const int s = 31 - __clz(i + 1), m = i + 1 - (1 << s);
         double sn, c;
         table_sincos((double)m * (pi_d / (double)(1 << s)), &sn, &c);
         tws[i] = mk(c, sn);
     }
-    if (tw && i < nhalf) {
+    if (table == 0 && tw && i < nhalf) {
         double sn, c;
         table_sincos((double)i * (pi_d / (double)nhalf), &sn, &c);
         tw[i] = mk(c, sn);
     }
-    if (filt && i < nbin) {
+    if (table == 1 && filt && i < nbin) {
         double v = 1.0;
         if (!(f.w1 == 0.0 && f.w2 == 0.0 && f.w3 == 0.0 && f.w4 == 0.0)) {
             const double w = __dmul_rn((double)i, f.df);
@@ -93,7 +94,7 @@ __global__ void k_time_tables(int nstage, cd* __restrict__ tws, int nhalf, cd* _
         }
         filt[i] = v;
     }
-    if (expt && i < nout) expt[i] = table_exp(ep * ((double)i * dt));
+    if (table == 2 && expt && i < nout) expt[i] = table_exp(ep * ((double)i * dt));
 }
 
 cudaError_t launch_time_tables(int nstage, cd* tws, int nhalf, cd* tw, const TaperDev& f, int nbin, double* filt,
@@ -105,7 +106,7 @@ cudaError_t launch_time_tables(int nstage, cd* tws, int nhalf, cd* tw, const Tap
     if (filt && nbin > n) n = nbin;
     if (expt && nout > n) n = nout;
     if (n == 0) return cudaSuccess;
-    k_time_tables<<<(n + 127) / 128, 128, 0, st>>>(nstage, tws, nhalf, tw, f, nbin, filt, ep, dt, nout, expt);
+    k_time_tables<<<dim3((n + 127) / 128, 3), 128, 0, st>>>(nstage, tws, nhalf, tw, f, nbin, filt, ep, dt, nout, expt);
     return cudaGetLastError();
 }
 
@@ -125,7 +126,7 @@ cudaError_t launch_time_tables(int nstage, cd* tws, int nhalf, cd* tw, const Tap
 // Positions are stored at p ^ ((p >> 3) & 7), so that 8 neighbouring threads
 // use different banks in every round, also in the first, where each has 8
 // consecutive values.  400 receivers, 1200 rows of 16384 and 7202 samples
-// kept: 257 us (the two passes in 16 MiB of rows, twiddles by sincos: 1286);
+// kept: 255 us (the two passes in 16 MiB of rows, twiddles by sincos: 1286);
 // half the issue slots are used, the rest wait for twiddles from the L2 and
 // at the rounds' barriers.  Tiles of 2048 take 5 us more (128 threads) or 100
 // (256), 512 threads on a tile 27.

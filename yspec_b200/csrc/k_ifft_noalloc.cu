@@ -20,7 +20,7 @@
 // host threads on the same device) race on it and must be serialised by the
 // caller.
 //
-// 400 receivers of 16384 samples: 257 us (k_series of k_ifft.cu; rows
+// 400 receivers of 16384 samples: 255 us (k_series of k_ifft.cu; rows
 // passed through the array, twiddles by sincos in every butterfly: 1286 us).
 //
 // The device address of the array is looked up with cudaGetSymbolAddress
